@@ -292,6 +292,7 @@ int fx_force_create(const fx_mesh* mesh, int32_t device, fx_force** out) {
         p.rho = q.rho;
         for (int d = 0; d < 3; ++d) p.b[d] = q.b[d];
         p.alphaM = q.alphaM;
+        s.any_alpha = s.any_alpha || q.alphaM != 0.0;
         p.betaK = q.betaK;
         p.betaKinit = q.betaKinit;
         p.betaKcomm = q.betaKcomm;

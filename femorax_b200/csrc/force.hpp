@@ -186,6 +186,7 @@ struct ForceState {
   DeviceArray<double> nodal_mass, nodal_alpha_mass, lumped_mass;
   DeviceArray<int8_t> eq_dof;
   bool has_nodal_mass = false, has_nodal_alpha = false;
+  bool any_alpha = false;  // a parameter set with mass-proportional damping
   int path = FX_PATH_AUTO;  // requested
   BoxPlan box;
   // work vectors (host-buffer apply, solvers)

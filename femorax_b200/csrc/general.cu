@@ -10,6 +10,7 @@
 #include <cstring>
 
 #include "force.hpp"
+#include "points.cuh"
 #include "ssp_brick.cuh"
 
 namespace fx {
@@ -68,6 +69,157 @@ __global__ void __launch_bounds__(kBlock) k_element_apply(const double* __restri
   else if (p.kind == 3) element_apply_d(p, f, xl, xe, ye, PdmyPointD{pdmy + p.table, dtan + e, dcs + e, P, f.cK, f.c0, f.cc});
   else element_apply(p, f, xl, xe, ye);
   for (int a = 0; a < 24; ++a) slots[static_cast<int64_t>(a) * P + e] = ye[a];
+}
+
+// The exact operator of elastic and J2 stdBrick sets, point-parallel (points.cuh): the same sums in
+// the same order as element_apply_d, so the same bits. A corner's value is the sum over the points,
+// in point order, of the point's stress term and then its mass term: each point leaves the two
+// (MASS) or one in shared memory, and 768 sums per block add them up.
+//
+// The elastic matrix's zero entries are left out of the stress sums where that gives the same value
+// (a finite strain: x + 0 e = x, and the sums start from +0), and a warp whose points all have the
+// elastic tangent (thetab = 0: the rank-one term is a signed zero) leaves out the rank-one term.
+__device__ __forceinline__ void sparse_stress(double l2m, double lam, double mu, const double e[6], double sg[6]) {
+  sg[0] = 0.0 + l2m * e[0] + lam * e[1] + lam * e[2];
+  sg[1] = 0.0 + lam * e[0] + l2m * e[1] + lam * e[2];
+  sg[2] = 0.0 + lam * e[0] + lam * e[1] + l2m * e[2];
+  sg[3] = 0.0 + mu * e[3];
+  sg[4] = 0.0 + mu * e[4];
+  sg[5] = 0.0 + mu * e[5];
+}
+
+template <bool MASS>
+__global__ void __launch_bounds__(points::kThreads, 2)
+    k_points_apply(const double* __restrict__ coords, const int32_t* __restrict__ node, const int32_t* __restrict__ eq,
+                   const int32_t* __restrict__ param, const ParamGP* __restrict__ params, int32_t N, int32_t P,
+                   int32_t count, double ks, double kd, double km, const double* __restrict__ x,
+                   double* __restrict__ slots, const int* skip, const double* __restrict__ j2tan, int initial) {
+  if (skip && *skip) return;
+  extern __shared__ __align__(16) unsigned char raw[];
+  auto& S = *reinterpret_cast<points::Stage<1, MASS ? 2 : 1>*>(raw);
+  points::stage_elements(S, coords, node, eq, N, P, count, x, nullptr);
+  const int gp = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int32_t e = static_cast<int32_t>(blockIdx.x) * points::kEl + l;
+  const bool ok = e < count;
+  {
+    const ParamGP& p = params[param[ok ? e : 0]];
+    const OpFactors f = op_factors(p, ks, kd, km, initial != 0);
+    const points::PointTable& tab = S.tab[gp];
+    double dN[3][8], dvol, ep[6], sg[6];
+    points::shape(S, tab, l, dN, dvol);
+    points::strain(dN, S.x[0], l, ep);
+    const double sum = ep[0] + ep[1] + ep[2] + ep[3] + ep[4] + ep[5];
+    bool sparse = fabs(sum) < INFINITY;
+    if (p.kind == 1) {  // J2PointD
+      const double cK = initial ? f.c0 : f.cK;
+      double theta = 1.0, thetab = 0.0;
+      const double* t = j2tan + e + static_cast<int64_t>(gp) * P;
+      const int64_t ld = 8 * static_cast<int64_t>(P);
+      if (!initial && ok) {
+        theta = t[0];
+        thetab = t[ld];
+      }
+      double K, G;
+      j2_moduli(p, K, G);
+      const double gt = 2.0 * G * theta;
+      sparse = sparse && thetab == 0.0 && fabs(gt) < INFINITY && fabs(cK) < INFINITY;
+      if (__all_sync(__activemask(), sparse)) {
+        sparse_stress(cK * (K + gt * (1.0 - 1.0 / 3.0)), cK * (K + gt * (0.0 - 1.0 / 3.0)), cK * (0.0 + gt * 0.5), ep, sg);
+      } else {
+        double n[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) n[c] = !initial && ok ? t[(2 + c) * ld] : 0.0;
+        const double gb = 2.0 * G * thetab;
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+          double s = 0.0;
+#pragma unroll
+          for (int c = 0; c < 6; ++c) {
+            const double idev = a < 3 && c < 3 ? (a == c ? 1.0 : 0.0) - 1.0 / 3.0 : (a == c ? 0.5 : 0.0);
+            const double vol = a < 3 && c < 3 ? K : 0.0;
+            const double D = vol + gt * idev - gb * n[a] * n[c];
+            s += cK * D * ep[c];
+          }
+          sg[a] = s;
+        }
+      }
+    } else {  // ConstD of effective_D
+      double l2m, lam, mu;
+      lame(p, l2m, lam, mu);
+      auto eff = [&](double d) {
+        double v = f.cK * d;
+        if (f.c0 != 0.0) v += f.c0 * d;
+        if (f.cc != 0.0) v += f.cc * d;
+        return v;
+      };
+      l2m = eff(l2m);
+      lam = eff(lam);
+      mu = eff(mu);
+      const double z = eff(0.0);  // NaN for an infinite factor
+      if (sparse && z == 0.0) {
+        sparse_stress(l2m, lam, mu, ep, sg);
+      } else {
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+          double s = 0.0;
+#pragma unroll
+          for (int c = 0; c < 6; ++c) s += (a < 3 && c < 3 ? (a == c ? l2m : lam) : (a == c ? mu : z)) * ep[c];
+          sg[a] = s;
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 6; ++c) sg[c] = sg[c] * dvol;
+    double vg[3] = {0.0, 0.0, 0.0};
+    if constexpr (MASS) {
+      if (p.mass_type == 0)
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+#pragma unroll
+          for (int q = 0; q < 3; ++q) vg[q] += tab.N[k] * S.x[0][3 * k + q][l];
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      double r[3];
+      points::corner_force(dN, sg, j, r);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) S.part[gp][0][3 * j + q][l] = r[q];
+      if constexpr (MASS) {
+        const double t = tab.N[j] * dvol * p.rho;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const double mj = t * (p.mass_type == 0 ? vg[q] : S.x[0][3 * j + q][l]);
+          S.part[gp][1][3 * j + q][l] = f.cM != 0.0 ? f.cM * mj : 0.0;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (!ok) return;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int a = gp + 8 * k;
+    double s = 0.0;
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      s += S.part[g][0][a][l];
+      if constexpr (MASS) s += S.part[g][1][a][l];
+    }
+    slots[static_cast<int64_t>(a) * P + e] = s;
+  }
+}
+
+template <bool MASS>
+void launch_points_apply(ForceState& s, const double k[3], const double* x, cudaStream_t st, const int* skip) {
+  constexpr int bytes = static_cast<int>(sizeof(points::Stage<1, MASS ? 2 : 1>));
+  static const bool once = [] {  // (thread-safe)
+    FX_CUDA(cudaFuncSetAttribute(k_points_apply<MASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    return true;
+  }();
+  (void)once;
+  k_points_apply<MASS><<<grid_for(s.count, points::kEl), points::kThreads, bytes, st>>>(
+      s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr, s.params.ptr, s.N, s.P, s.count, k[0], k[1], k[2], x,
+      s.slots.ptr, skip, s.j2_tan.ptr, s.initial);
 }
 
 __global__ void __launch_bounds__(kBlock) k_element_diag(const double* __restrict__ coords, const int32_t* __restrict__ node,
@@ -454,17 +606,39 @@ __device__ __forceinline__ T slot_sum(const int32_t* __restrict__ list, const T*
 }
 
 // The same sum by one warp, for equations with many slots (a tied DOF gathers whole rows of
-// elements): 32 slots loaded at once, then added in list order by every lane.
+// elements): 256 slots loaded at once, the next 256 on their way while these are added in list order
+// by every lane. The 640 slots of a tied DOF of the 40^3 laminar column are then one chain of
+// additions: the gather launch takes 17 us there instead of 33 (32 slots at a time, each batch
+// waiting for its list entries and then its slots).
 template <class T>
 __device__ __forceinline__ T slot_sum_warp(const int32_t* __restrict__ list, const T* __restrict__ slots, int32_t j0,
                                            int32_t j1) {
+  constexpr int U = 8;
   const int lane = threadIdx.x & 31;
+  auto fetch = [&](int32_t b, T (&v)[U]) {  // slots b + 32 u + lane of the list (0 past its end)
+    int32_t idx[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) idx[u] = b + 32 * u + lane < j1 ? list[b + 32 * u + lane] : -1;
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = idx[u] >= 0 ? slots[idx[u]] : T(0);
+  };
+  T v[U], next[U];
   T sum = T(0);
-  for (int32_t b = j0; b < j1; b += 32) {
-    const int32_t j = b + lane;
-    const T v = j < j1 ? slots[list[j]] : T(0);
-    const int cnt = j1 - b < 32 ? j1 - b : 32;
-    for (int u = 0; u < cnt; ++u) sum += __shfl_sync(0xffffffffu, v, u);
+  fetch(j0, v);
+  for (int32_t b = j0; b < j1; b += 32 * U) {
+    if (b + 32 * U < j1) fetch(b + 32 * U, next);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int cnt = min(32, j1 - b - 32 * u);
+      if (cnt == 32) {
+#pragma unroll
+        for (int k = 0; k < 32; ++k) sum += __shfl_sync(0xffffffffu, v[u], k);
+      } else {
+        for (int k = 0; k < cnt; ++k) sum += __shfl_sync(0xffffffffu, v[u], k);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = next[u];
   }
   return sum;
 }
@@ -929,13 +1103,17 @@ void general_force_gather(ForceState& s, const double* v, double* f, cudaStream_
 void general_apply(ForceState& s, const double k[3], const double* x, double* y, cudaStream_t st, const int* skip) {
   refuse_pimy_initial(s);
   if (general_fast_applies(s)) return general_apply_fast(s, k, x, y, st, skip);
-  if (s.count > 0)
+  if (s.count > 0 && !s.has_ssp && !s.has_pimy && !s.has_pdmy) {  // every set an elastic or J2 stdBrick set
+    if (k[2] != 0.0 || (k[1] != 0.0 && s.any_alpha)) launch_points_apply<true>(s, k, x, st, skip);
+    else launch_points_apply<false>(s, k, x, st, skip);
+  } else if (s.count > 0) {
     k_element_apply<<<grid_for(s.count, kBlock), kBlock, 0, st>>>(s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr,
                                                                    s.params.ptr, s.N, s.P, s.count, k[0], k[1], k[2],
                                                                    -1, x, s.slots.ptr, skip, s.j2_tan.ptr, s.initial,
                                                                    s.pimy_dev.ptr, s.pimy_tan.ptr, s.pdmy_dev.ptr,
                                                                    s.pdmy_tan.ptr, s.pimy_committed.ptr,
                                                                    s.pdmy_committed.ptr, s.ssp_geo.ptr, s.ssp_con.ptr);
+  }
   FX_LAUNCH_CHECK("element_apply");
   const double* m1 = (k[2] != 0.0 && s.has_nodal_mass) ? s.nodal_mass.ptr : nullptr;
   const double* m2 = (k[1] != 0.0 && s.has_nodal_alpha) ? s.nodal_alpha_mass.ptr : nullptr;
