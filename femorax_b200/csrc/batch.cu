@@ -569,6 +569,7 @@ struct Engine {
   DeviceArray<unsigned char> inst64i;         // FP64 inner solves: the inner apply's descriptors
   DeviceArray<int4> work;
   int nwork = 0;
+  int kz = 8;  // node planes per work item's tile
   DeviceArray<int> queue;  // [next item, CTAs done] of the persistent batched apply, zero between launches
   // The batched apply as one CTA per work item (the default: 0.480-0.485 s against 0.501 s for the
   // persistent wave on 120 static solves with FP32 inner solves, equal with FP64 ones, B200) or as a
@@ -623,11 +624,15 @@ struct Engine {
         sdh[s] = SlotDev{slots[s].c0 * kChunk, slots[s].n, slots[s].c0, slots[s].nc};
         high = std::max(high, slots[s].c0 + slots[s].nc);
       }
+    std::vector<const ForceState*> grids;
+    for (int s = 0; s < max_slots; ++s)
+      if (slots[s].used && !fl_h[s * NFL + G_FIN]) grids.push_back(&slots[s].f->s);
+    kz = box_batch_planes(grids, !inner64);  // (the inner iterations' launch)
     std::vector<int4> wl;
     for (int s = 0; s < max_slots; ++s) {
       if (!slots[s].used || fl_h[s * NFL + G_FIN]) continue;
       int gx, gy, gz;
-      box_batch_tiles(slots[s].f->s, gx, gy, gz);
+      box_batch_tiles(slots[s].f->s, kz, gx, gy, gz);
       for (int z = 0; z < gz; ++z)
         for (int y = 0; y < gy; ++y)
           for (int xx = 0; xx < gx; ++xx) wl.push_back(make_int4(s, xx, y, z));
@@ -657,7 +662,7 @@ struct Engine {
 
   template <class TI>
   void inner_iteration_t(const unsigned char* inst, TI* p, TI* ap, const TI* iv, TI* d, TI* rr) {
-    box_batch_apply(sizeof(TI) == 4, inst, work.ptr, nwork, persistent ? queue.ptr : nullptr, cs);
+    box_batch_apply(sizeof(TI) == 4, inst, work.ptr, nwork, kz, persistent ? queue.ptr : nullptr, cs);
     if (high <= kBlockChunks) {  // a block per chunk
       const unsigned gb = static_cast<unsigned>(high);
       k_b_pap<TI, true><<<gb, kChunkBlock, 0, cs>>>(p, ap, high, nchunks, chunk_slot.ptr, sd_dev.ptr, fl.ptr, o.lanes,
@@ -724,7 +729,7 @@ struct Engine {
     }
     if (any_outer) {  // the slots due for it: r = b - K x (FP64), norms, test, the inner solve's start
       k_b_phase<<<slot_grid(), 128, 0, cs>>>(fl.ptr, used_dev.ptr, max_slots);
-      box_batch_apply(false, inst64.ptr, work.ptr, nwork, persistent ? queue.ptr : nullptr, cs);
+      box_batch_apply(false, inst64.ptr, work.ptr, nwork, kz, persistent ? queue.ptr : nullptr, cs);
       k_b_residual<<<g, 32 * kWarps, 0, cs>>>(b.ptr, ap.ptr, r.ptr, high, chunk_slot.ptr, sd_dev.ptr, fl.ptr, o.lanes,
                                               part.ptr, nchunks);
       level(2, G_SKIP, O_RR);

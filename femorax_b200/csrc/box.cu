@@ -434,9 +434,22 @@ void box_force_f32(ForceState& s, const float* u, const float* v, float* f, cuda
   force_t<float>(s, u, v, f, st);
 }
 
-// Meshes below this many elements take the launch shape that is fastest on large grids (16 x 8
-// columns, 8 planes) without timing.
+// Meshes below this many elements take 16 x 8 columns without timing, and as few planes per tile as
+// keep the tiles in one wave.
 constexpr int32_t kTuneMinElements = 262144;
+
+// Planes per tile of a grid that is not timed. A tile is a serial sweep up its planes, about 1.1 us
+// each after 2.5 us of launch and prologue, so while SMs would stand idle more and shorter tiles are
+// faster, and past one wave of resident CTAs (4 per SM, 3 with two staged vectors) they are not.
+// Apply, B200, FP64 (FP32 within 10 %), 8 planes against this rule: 5^3 8.8 -> 3.7 us (1 plane),
+// 32^3 12.0 -> 6.2 (1), 44^3 13.4 -> 9.5 (2; 11.6 with 1, 1.6 waves), 60 x 60 x 50 15.0 -> 12.5 (4,
+// 585 tiles; 14.6 with 3).
+int one_wave_planes(const BoxPlan& p, int ctas_per_sm) {
+  const int64_t cols = static_cast<int64_t>((p.nx + 1 + 14) / 15) * ((p.ny + 1 + 6) / 7);
+  for (int kz = 1; kz < 8; ++kz)
+    if (cols * ((p.nz + 1 + kz - 1) / kz) <= static_cast<int64_t>(ctas_per_sm) * num_sms()) return kz;
+  return 8;
+}
 
 // Times every launch variant and plane count, as a grid and as a persistent launch, on the operator
 // (unit stiffness) and, where the box force form applies, on the internal force, each in FP64 and
@@ -446,7 +459,7 @@ void box_autotune(ForceState& s, cudaStream_t st) {
   if (!s.box.qualifies) return;
   if (s.count < kTuneMinElements) {  // launch-bound: timing costs more than it can save
     for (auto& per_mode : s.box.shape)
-      for (auto& sh : per_mode) sh = BoxPlan::Shape{};
+      for (int mode = 0; mode < 2; ++mode) per_mode[mode] = BoxPlan::Shape{2, one_wave_planes(s.box, mode == 1 ? 3 : 4), false};
     s.box.tuned = true;
     return;
   }
@@ -522,26 +535,35 @@ void box_autotune(ForceState& s, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ batches of grids
-// One launch shape for batches: 16 x 8 element columns, 4 CTAs per SM (FP64) or 6 (FP32), kBatchKz
-// node planes per tile.
+// One launch shape for batches: 16 x 8 element columns, 4 CTAs per SM (FP64) or 6 (FP32); the node
+// planes per tile are the caller's (one work list, one count).
 namespace {
-constexpr int kBatchBX = 16, kBatchBY = 8, kBatchKz = 8;
+constexpr int kBatchBX = 16, kBatchBY = 8;
 template <class T>
 constexpr int kBatchMinB = sizeof(T) == 4 ? 6 : 4;  // FP32 fits 6 CTAs per SM without spills
 
+// CTAs of the batch kernel that are resident at once (set once, thread-safe: serving threads launch
+// this concurrently)
 template <class T>
-void batch_launch(const void* inst, const int4* work, int nwork, int* queue, cudaStream_t st) {
+int batch_resident() {
   using S = Smem<kBatchBX, kBatchBY, T, 0, kPerSet>;
   auto kern = k_box_batch<kBatchBX, kBatchBY, T, 0, kBatchMinB<T>>;
-  // CTAs per SM (set once, thread-safe: serving threads launch this concurrently)
   static const int resident = [&] {
     int r = 0;
     FX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(S::bytes)));
     FX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kern, kBatchBX * kBatchBY, S::bytes));
-    return std::max(r, 1);
+    return std::max(r, 1) * num_sms();
   }();
-  const int ctas = queue ? std::min(nwork, resident * num_sms()) : nwork;
-  kern<<<ctas, kBatchBX * kBatchBY, S::bytes, st>>>(static_cast<const BoxArgs<T>*>(inst), work, nwork, queue);
+  return resident;
+}
+
+template <class T>
+void batch_launch(const void* inst, const int4* work, int nwork, int kz, int* queue, cudaStream_t st) {
+  using S = Smem<kBatchBX, kBatchBY, T, 0, kPerSet>;
+  auto kern = k_box_batch<kBatchBX, kBatchBY, T, 0, kBatchMinB<T>>;
+  const int resident = batch_resident<T>();
+  const int ctas = queue ? std::min(nwork, resident) : nwork;
+  kern<<<ctas, kBatchBX * kBatchBY, S::bytes, st>>>(static_cast<const BoxArgs<T>*>(inst), work, nwork, kz, queue);
   FX_LAUNCH_CHECK("box_batch");
 }
 
@@ -549,7 +571,6 @@ template <class T>
 void fill_args(ForceState& s, const double k[3], const void* x, void* y, const int* skip, void* dst) {
   ensure_coef(s, 0, k);
   BoxArgs<T> a = args<T>(s, 0, static_cast<const T*>(x), nullptr, static_cast<T*>(y));
-  a.kz = kBatchKz;
   a.skip = skip;
   if (k[2] != 0.0 && s.has_nodal_mass) {
     a.nm1 = s.nodal_mass.ptr;
@@ -734,16 +755,30 @@ void box_fill_args(ForceState& s, const double k[3], bool f32, const void* x, vo
   else fill_args<double>(s, k, x, y, skip, dst);
 }
 
-void box_batch_tiles(const ForceState& s, int& gx, int& gy, int& gz) {
+void box_batch_tiles(const ForceState& s, int kz, int& gx, int& gy, int& gz) {
   gx = (s.box.nx + 1 + kBatchBX - 2) / (kBatchBX - 1);
   gy = (s.box.ny + 1 + kBatchBY - 2) / (kBatchBY - 1);
-  gz = (s.box.nz + 1 + kBatchKz - 1) / kBatchKz;
+  gz = (s.box.nz + 1 + kz - 1) / kz;
 }
 
-void box_batch_apply(bool f32, const void* inst, const int4* work, int nwork, int* queue, cudaStream_t st) {
+int box_batch_planes(const std::vector<const ForceState*>& grids, bool f32) {
+  const int64_t resident = f32 ? batch_resident<float>() : batch_resident<double>();
+  for (int kz = 1; kz < 8; ++kz) {
+    int64_t items = 0;
+    for (const ForceState* s : grids) {
+      int gx, gy, gz;
+      box_batch_tiles(*s, kz, gx, gy, gz);
+      items += static_cast<int64_t>(gx) * gy * gz;
+    }
+    if (items <= resident) return kz;
+  }
+  return 8;
+}
+
+void box_batch_apply(bool f32, const void* inst, const int4* work, int nwork, int kz, int* queue, cudaStream_t st) {
   if (nwork <= 0) return;
-  if (f32) batch_launch<float>(inst, work, nwork, queue, st);
-  else batch_launch<double>(inst, work, nwork, queue, st);
+  if (f32) batch_launch<float>(inst, work, nwork, kz, queue, st);
+  else batch_launch<double>(inst, work, nwork, kz, queue, st);
 }
 
 }  // namespace fx

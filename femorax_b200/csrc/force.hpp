@@ -312,9 +312,11 @@ bool box_apply_host(ForceState& s, const double k[3], const double* xh, double* 
 // (grid, tile x, tile y, tile z) items.
 size_t box_args_bytes(bool f32);
 void box_fill_args(ForceState& s, const double k[3], bool f32, const void* x, void* y, const int* skip, void* dst);
-void box_batch_tiles(const ForceState& s, int& gx, int& gy, int& gz);
+void box_batch_tiles(const ForceState& s, int kz, int& gx, int& gy, int& gz);
+// node planes per tile of a batch of these grids: as few as keep its items in one wave, at most 8
+int box_batch_planes(const std::vector<const ForceState*>& grids, bool f32);
 // queue: a device int[2], zero between launches, for the persistent form (NULL: one CTA per item)
-void box_batch_apply(bool f32, const void* inst, const int4* work, int nwork, int* queue, cudaStream_t st);
+void box_batch_apply(bool f32, const void* inst, const int4* work, int nwork, int kz, int* queue, cudaStream_t st);
 
 }  // namespace fx
 
