@@ -27,6 +27,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cg_fused.cuh"
 #include "force.hpp"
 #include "vector.hpp"
 
@@ -53,7 +54,8 @@ enum : int {
   G_OUTER, G_INNER, G_INNER_RAN,
   G_NEED_OUTER,  // due for an outer step (admitted, or corrected and not finished)
   F_BEGIN,       // its inner solve starts in this tick (set by the outer step)
-  NFL = 13
+  F_GAVE_UP,     // a block did not reach a reduction of the fused iteration
+  NFL = 14
 };
 
 struct SlotDev {
@@ -488,6 +490,47 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// The three kernels of an inner iteration in one cooperative launch (cg_fused.cuh), a block per chunk
+// up to the highest in use; the blocks of one slot meet at its two reductions (bar: two counters per
+// slot) and its first block keeps its scalars. part: three columns, ld apart.
+template <class TI>
+__global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<TI>)
+    k_b_fused(double* sc, int* fl, TI* p, const TI* ap, const TI* inv, TI* d, TI* rr,
+              const int* __restrict__ chunk_slot, const SlotDev* __restrict__ sd, int lanes, double* part, int64_t ld,
+              unsigned long long* bar) {
+  const int64_t c = blockIdx.x, begin = c * kChunk;
+  const int s = slot_of_chunk(chunk_slot, c);
+  if (s < 0 || fl[s * NFL + F_DONE]) return;  // (the same for the slot's blocks)
+  int* f = fl + s * NFL;
+  double* cs = sc + s * NSC;
+  const SlotDev S = sd[s];
+  const int64_t left = S.off + S.n - begin;
+  const int it = f[F_ITERS];
+  cgf::Chunk<TI> a{p, ap, inv, d, rr, begin, static_cast<int>(left < kChunk ? left : kChunk), lanes, c - S.c0, S.nc,
+                   part + S.c0, ld, bar + 2 * s, cs[S_RZ], cs[S_TOL], it, f[F_MAXIT]};
+  const cgf::Sums o = cgf::iterate(a);
+  if (o.state == cgf::kGaveUp && threadIdx.x == 0) f[F_GAVE_UP] = f[F_DONE] = 1;
+  if (a.c != 0 || threadIdx.x != 0 || o.state == cgf::kGaveUp) return;
+  cs[S_PAP] = o.pap;
+  if (o.state == cgf::kIndefinite) {
+    f[F_INDEF] = 1;
+    f[F_DONE] = 1;
+    return;
+  }
+  cs[S_ALPHA] = a.rz / o.pap;
+  cs[S_RR] = o.rr;
+  cs[S_RZNEW] = o.rz;
+  cs[S_RNORM] = sqrt(o.rr);
+  f[F_ITERS] = it + 1;
+  if (o.state == cgf::kConverged) f[F_CONV] = 1;
+  if (o.state != cgf::kGoOn) {
+    f[F_DONE] = 1;
+    return;
+  }
+  cs[S_BETA] = o.rz / a.rz;
+  cs[S_RZ] = o.rz;
+}
+
 // x += (double) d for slots that ran an inner solve this round; the round's counters
 template <class TI>
 __global__ void __launch_bounds__(32 * kWarps)
@@ -560,7 +603,8 @@ struct Engine {
   bool inner64 = false;
   DeviceArray<double> r64, d64, rr64, p64, ap64;
   DeviceArray<int> chunk_slot;
-  DeviceArray<double> part;  // [2][nchunks]
+  DeviceArray<double> part;  // [3][nchunks]
+  DeviceArray<unsigned long long> meet;  // per slot: the fused iteration's two meetings (0 at admission)
   DeviceArray<double> sc;
   DeviceArray<int> fl, used_dev, zeros;
   DeviceArray<unsigned> cnt;  // per slot: chunks counted by the fused reductions (0 between launches)
@@ -663,7 +707,11 @@ struct Engine {
   template <class TI>
   void inner_iteration_t(const unsigned char* inst, TI* p, TI* ap, const TI* iv, TI* d, TI* rr) {
     box_batch_apply(sizeof(TI) == 4, inst, work.ptr, nwork, kz, persistent ? queue.ptr : nullptr, cs);
-    if (high <= kBlockChunks) {  // a block per chunk
+    static const int64_t fused_chunks = cgf::capacity(k_b_fused<TI>);  // (thread-safe)
+    if (high <= fused_chunks) {  // one launch, every chunk resident
+      cgf::launch(k_b_fused<TI>, high, cs, sc.ptr, fl.ptr, p, ap, iv, d, rr, chunk_slot.ptr, sd_dev.ptr, o.lanes,
+                  part.ptr, nchunks, meet.ptr);
+    } else if (high <= kBlockChunks) {  // a block per chunk
       const unsigned gb = static_cast<unsigned>(high);
       k_b_pap<TI, true><<<gb, kChunkBlock, 0, cs>>>(p, ap, high, nchunks, chunk_slot.ptr, sd_dev.ptr, fl.ptr, o.lanes,
                                                     part.ptr, sc.ptr, cnt.ptr);
@@ -766,6 +814,9 @@ struct Engine {
     }
     FX_CUDA(cudaGraphLaunch(graph, cs));
     read_flags();
+    for (int s = 0; s < max_slots; ++s)
+      if (slots[s].used && fl_h[s * NFL + F_GAVE_UP])
+        throw Error(FX_E_TIMEOUT, "batched CG: a block did not reach its slot's reduction");
     // slots that finished leave the work list
     for (int s = 0; s < max_slots; ++s)
       if (slots[s].used && fl_h[s * NFL + G_FIN]) dirty = true;
@@ -830,6 +881,7 @@ struct Engine {
     std::vector<double> s0(NSC, 0.0);
     FX_CUDA(cudaMemcpyAsync(fl.ptr + slot * NFL, f0.data(), sizeof(int) * NFL, cudaMemcpyHostToDevice, cs));
     FX_CUDA(cudaMemcpyAsync(sc.ptr + slot * NSC, s0.data(), sizeof(double) * NSC, cudaMemcpyHostToDevice, cs));
+    FX_CUDA(cudaMemsetAsync(meet.ptr + 2 * slot, 0, 2 * sizeof(unsigned long long), cs));
     FX_CUDA(cudaStreamSynchronize(cs));
     if (nz > 0) {
       // leave the range free again: nothing points at it
@@ -918,7 +970,9 @@ int fx_engine_create(int32_t device, int64_t capacity, int32_t max_slots, fx_coe
       for (auto* v : {&e.b, &e.x, &e.r, &e.ap, &e.inv}) v->alloc(n);
       for (auto* v : {&e.r32, &e.d32, &e.rr32, &e.p32, &e.ap32, &e.inv32}) v->alloc(n);
       e.chunk_slot.alloc(static_cast<size_t>(e.nchunks));
-      e.part.alloc(static_cast<size_t>(e.nchunks) * 2);
+      e.part.alloc(static_cast<size_t>(e.nchunks) * 3);
+      e.meet.alloc(static_cast<size_t>(max_slots) * 2);
+      FX_CUDA(cudaMemset(e.meet.ptr, 0, e.meet.bytes()));
       e.sc.alloc(static_cast<size_t>(max_slots) * fx::NSC);
       e.fl.alloc(static_cast<size_t>(max_slots) * fx::NFL);
       e.used_dev.alloc(static_cast<size_t>(max_slots));

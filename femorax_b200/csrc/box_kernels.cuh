@@ -237,7 +237,7 @@ __device__ __forceinline__ void box_tile(const BoxArgs<T>& a, const BoxTable<typ
   T* yo = xs + NB * NV * 3 * NS;                            // [2][3][NO]: owned nodes' sums
   int32_t* es = reinterpret_cast<int32_t*>(yo + 6 * NO);   // [NB][NS]: equations
   int32_t* yq = es + NB * NS;                               // [2][NO]: owned nodes' equations (0: none)
-  if (a.skip && *a.skip) return;
+  const int skip = a.skip ? *a.skip : 0;  // (its load overlaps the prologue's)
 
   const int t = threadIdx.x;
   const int ci = t % BX, cj = t / BX;
@@ -384,6 +384,7 @@ __device__ __forceinline__ void box_tile(const BoxArgs<T>& a, const BoxTable<typ
   for (int k = k0 - 1; k <= k0 + D; ++k) copy_equations(k, k - k0 + 1);
   cp_async_commit();
   cp_async_wait<0>();
+  if (skip) return;
   __syncthreads();  // the values' copies read other threads' equations
   for (int k = k0 - 1; k <= k0 + D - 2; ++k) copy_values(k, k - k0 + 1);
   cp_async_commit();

@@ -15,6 +15,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cg_fused.cuh"
 #include "force.hpp"
 #include "vector.hpp"
 
@@ -43,6 +44,7 @@ enum : int {
   G_IR_OUTER,         // refinement rounds of this linear solve
   G_IR_INNER,         // inner iterations of this linear solve
   G_IR_REFS,          // refinement rounds in all
+  G_GAVE_UP,          // a block did not reach a reduction of the fused iteration
   NNF = 16
 };
 
@@ -447,6 +449,44 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// The three kernels of a CG iteration in one cooperative launch (cg_fused.cuh), a block per chunk of
+// the combined vectors; the blocks of one instance meet at its two reductions (bar: two counters per
+// instance) and its first block keeps its scalars. part: three columns of nchunks sums.
+template <class T>
+__global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<T>)
+    k_nb_fused(double* sc, int* fl, T* p, const T* ap, const T* inv, T* du, T* rr, const int* __restrict__ owner,
+               const Range* __restrict__ rg, int lanes, double* part, unsigned long long* bar) {
+  const int64_t c = blockIdx.x, begin = c * kChunk;
+  const int s = owner[c];
+  if (s < 0 || fl[s * NNF + G_CG_DONE]) return;  // (the same for the instance's blocks)
+  int* f = fl + s * NNF;
+  double* cs = sc + s * NNS;
+  const Range r = rg[s];
+  const int it = f[G_CG_ITERS];
+  cgf::Chunk<T> a{p, ap, inv, du, rr, begin, static_cast<int>(chunk_len(r, begin)), lanes, c - r.c0, r.nc,
+                  part + r.c0, gridDim.x, bar + 2 * s, cs[N_RZ], cs[N_TOL], it, f[G_CG_MAXIT]};
+  const cgf::Sums o = cgf::iterate(a);
+  if (o.state == cgf::kGaveUp && threadIdx.x == 0) f[G_GAVE_UP] = f[G_CG_DONE] = 1;
+  if (a.c != 0 || threadIdx.x != 0 || o.state == cgf::kGaveUp) return;
+  cs[N_PAP] = o.pap;
+  if (o.state == cgf::kIndefinite) {
+    f[G_INDEF] = 1;
+    f[G_CG_DONE] = 1;
+    return;
+  }
+  cs[N_ALPHA] = a.rz / o.pap;
+  cs[N_RR] = o.rr;
+  cs[N_RZNEW] = o.rz;
+  f[G_CG_ITERS] = it + 1;
+  if (o.state == cgf::kConverged) f[G_CG_CONV] = 1;
+  if (o.state != cgf::kGoOn) {
+    f[G_CG_DONE] = 1;
+    return;
+  }
+  cs[N_BETA] = o.rz / a.rz;
+  cs[N_RZ] = o.rz;
+}
+
 // u += du for instances that solved this iteration; their counters
 __global__ void __launch_bounds__(32 * kWarps)
     k_nb_correct(const double* __restrict__ du, double* __restrict__ u, int64_t nchunks,
@@ -630,6 +670,7 @@ struct NBatch {
   DeviceArray<double> r, du, rr, p, ap, d, inv, zero, part, sc;
   DeviceArray<int> fl;
   DeviceArray<unsigned> cnt;  // per instance: chunks counted by the fused reductions (0 between launches)
+  DeviceArray<unsigned long long> meet;  // per instance: the fused iteration's two meetings
   DeviceArray<int> passes;    // the CG loop graph's pass count
   int* fl_h = nullptr;
   double* sc_h = nullptr;
@@ -656,6 +697,10 @@ struct NBatch {
     FX_CUDA(cudaMemcpyAsync(fl_h, fl.ptr, sizeof(int) * NNF * count, cudaMemcpyDeviceToHost, cs));
     FX_CUDA(cudaMemcpyAsync(sc_h, sc.ptr, sizeof(double) * NNS * count, cudaMemcpyDeviceToHost, cs));
     FX_CUDA(cudaStreamSynchronize(cs));
+    if (any(G_GAVE_UP, 1)) {
+      FX_CUDA(cudaMemset(meet.ptr, 0, meet.bytes()));
+      throw Error(FX_E_TIMEOUT, "batched CG: a block did not reach its instance's reduction");
+    }
   }
   unsigned inst_grid() const { return static_cast<unsigned>((count + 127) / 128); }
   void level(int ncol, int gate, int dst) {
@@ -668,7 +713,11 @@ struct NBatch {
   // the vector kernels of one CG iteration (in vectors of type T), in the form for this many chunks
   template <class T>
   void cg_vectors(T* pv, T* apv, const T* iv, T* dv, T* rv) {
-    if (nchunks <= kBlockChunks) {  // a block per chunk
+    static const int64_t fused_chunks = cgf::capacity(k_nb_fused<T>);  // (thread-safe)
+    if (nchunks <= fused_chunks) {  // one launch, every chunk resident
+      cgf::launch(k_nb_fused<T>, nchunks, cs, sc.ptr, fl.ptr, pv, apv, iv, dv, rv, owner.ptr, rg.ptr, o.lanes,
+                  part.ptr, meet.ptr);
+    } else if (nchunks <= kBlockChunks) {  // a block per chunk
       const unsigned gb = static_cast<unsigned>(nchunks);
       k_nb_pap<T, true><<<gb, kChunkBlock, 0, cs>>>(pv, apv, nchunks, owner.ptr, rg.ptr, fl.ptr, o.lanes, part.ptr,
                                                     sc.ptr, cnt.ptr);
@@ -953,11 +1002,13 @@ int fx_nbatch_create(const fx_mesh* meshes, int32_t count, int32_t device, fx_so
         v->alloc(static_cast<size_t>(Q));
         v->zero(nullptr);
       }
-      b.part.alloc(static_cast<size_t>(b.nchunks) * 2);
+      b.part.alloc(static_cast<size_t>(b.nchunks) * 3);
       b.sc.alloc(static_cast<size_t>(count) * fx::NNS);
       b.fl.alloc(static_cast<size_t>(count) * fx::NNF);
       b.cnt.alloc(static_cast<size_t>(count));
       b.cnt.zero(nullptr);
+      b.meet.alloc(static_cast<size_t>(count) * 2);
+      b.meet.zero(nullptr);
       b.passes.alloc(1);
       FX_CUDA(cudaMallocHost(&b.fl_h, sizeof(int) * fx::NNF * count));
       FX_CUDA(cudaMallocHost(&b.sc_h, sizeof(double) * fx::NNS * count));

@@ -2,11 +2,11 @@
 // src/solvers/linear_solver.hpp:96-105, cg.cpp:24-71, gmres.cpp:32-123, krylov.cpp:25-41,
 // jacobi.cpp:10-26), B200-resident.
 //
-// CG keeps its scalars on the device: one iteration is the operator, the p.Ap reduction, a
-// one-thread kernel for alpha, one fused pass that updates x and r and forms the chunk sums of
-// r.r and r.z (z = D^-1 r, never stored), the reduction levels, a one-thread kernel for the
-// convergence test and beta, and the p update. The iterations run as a CUDA graph; the host
-// reads the `done` flag after each block of iterations. Every kernel returns at once when the
+// CG keeps its scalars on the device: one iteration is the operator and, where the vectors' chunks all
+// fit on the GPU at once, one cooperative launch for the rest (cg_fused.cuh); for longer vectors three
+// kernels: p.Ap with its levels and alpha, the update of x and r with r.r, r.z (z = D^-1 r, never
+// stored), their levels, the test and beta, and the p update. The iterations run as a CUDA graph with
+// a device-side loop; the host reads the `done` flag once per solve. Every kernel returns at once when the
 // solve is done, so the iterate is frozen at the converged one. All reductions use the
 // documented chunk/lane order (fused multiply-adds), so a solve gives the same bits every run.
 #include <functional>
@@ -15,6 +15,7 @@
 #include <cmath>
 #include <vector>
 
+#include "cg_fused.cuh"
 #include "force.hpp"
 #include "vector.hpp"
 
@@ -33,7 +34,7 @@ enum : int {
   S_BB = 10,
   S_NSCALAR = 16
 };
-enum : int { F_DONE = 0, F_CONV = 1, F_INDEF = 2, F_ITERS = 3, F_NFLAG = 4 };
+enum : int { F_DONE = 0, F_CONV = 1, F_INDEF = 2, F_ITERS = 3, F_GAVE_UP = 4, F_NFLAG = 5 };
 
 namespace fx {
 namespace {
@@ -336,6 +337,7 @@ __global__ void k_cg_start(double* sc, int* fl, double rtol, double atol, int ma
   sc[S_TOL] = tol > atol ? tol : atol;
   fl[F_ITERS] = 0;
   fl[F_INDEF] = 0;
+  fl[F_GAVE_UP] = 0;
   fl[F_CONV] = rn <= sc[S_TOL];
   fl[F_DONE] = fl[F_CONV] || max_it <= 0;
 }
@@ -369,9 +371,63 @@ __device__ void cg_beta_step(double* sc, int* fl, int max_it) {
   sc[S_RZ] = sc[S_RZNEW];
 }
 
-// CG iterations per pass of the loop graph: fewer condition kernels and body relaunches against
+// CG iterations per pass of the loop graph: fewer body relaunches (11.8 ms a 32^3 solve with 8, 12.1 with
+// 4, 12.7 with 2, before the fused iteration's arrivals were moved) and condition kernels against
 // at most kCgPass - 1 empty iterations after the solve ends.
-constexpr int kCgPass = 4;
+constexpr int kCgPass = 8;
+
+// The loop graph's condition as the fused iteration sets it (after the last iteration of a pass).
+struct PassEnd {
+  cudaGraphConditionalHandle h;
+  int* passes;
+  int cap;  // 0: not the last iteration of a pass
+};
+
+// k_cg_pap, k_cg_update and k_cg_p of one iteration in one cooperative launch (cg_fused.cuh), a block
+// per chunk, for vectors whose chunks all fit on the GPU at once; the first block keeps the scalars,
+// and, at the end of a pass, the loop's condition (k_cg_cond).
+template <class T>
+__global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<T>)
+    k_cg_fused(double* sc, int* fl, T* p, const T* ap, const T* inv, T* x, T* r, int64_t n, int lanes, double* part,
+               unsigned long long* bar, int max_it, PassEnd end) {
+  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  if (fl[F_DONE]) {  // (the same for every block: it changes after their last meeting only)
+    if (lead && end.cap) cudaGraphSetConditional(end.h, 0u);
+    return;
+  }
+  const int64_t c = blockIdx.x, nc = gridDim.x, begin = c * kChunk;
+  const int it = fl[F_ITERS];
+  cgf::Chunk<T> a{p, ap, inv, x, r, begin, static_cast<int>(n - begin < kChunk ? n - begin : kChunk), lanes, c, nc,
+                  part, nc, bar, sc[S_RZ], sc[S_TOL], it, max_it};
+  const cgf::Sums o = cgf::iterate(a);
+  if (o.state == cgf::kGaveUp && threadIdx.x == 0) {
+    fl[F_GAVE_UP] = 1;
+    fl[F_DONE] = 1;
+  }
+  if (!lead) return;
+  sc[S_PAP] = o.pap;
+  if (o.state == cgf::kIndefinite) {
+    fl[F_INDEF] = 1;
+    fl[F_DONE] = 1;
+  } else if (o.state != cgf::kGaveUp) {
+    sc[S_ALPHA] = a.rz / o.pap;
+    sc[S_RR] = o.rr;
+    sc[S_RZNEW] = o.rz;
+    sc[S_RNORM] = sqrt(o.rr);
+    fl[F_ITERS] = it + 1;
+    if (o.state == cgf::kConverged) fl[F_CONV] = 1;
+    if (o.state != cgf::kGoOn) {
+      fl[F_DONE] = 1;
+    } else {
+      sc[S_BETA] = o.rz / a.rz;
+      sc[S_RZ] = o.rz;
+    }
+  }
+  if (end.cap) {
+    const int passes = ++*end.passes;
+    cudaGraphSetConditional(end.h, o.state == cgf::kGoOn && passes < end.cap ? 1u : 0u);
+  }
+}
 
 // The condition of the CG loop graph: another pass while the solve is not done, at most `cap`
 // passes (a bound the solve's own max_it already keeps below).
@@ -469,6 +525,8 @@ struct Solver {
   DeviceArray<int> zero_count;
   DeviceArray<int> passes;  // the CG loop graph's pass counter
   DeviceArray<unsigned> counter;  // the fused kernels' last-block counter (0 between launches)
+  DeviceArray<double> fpart;              // the fused iteration's chunk sums, three columns
+  DeviceArray<unsigned long long> meet;   // and its two meetings' counters
   DeviceArray<double> V, Z, wv, hbuf;  // GMRES
   DeviceArray<double> nres, ndu;       // Newton: residual and increment
   DeviceArray<double> nut, nvt, nat;   // Newmark: the last step's u, v, a
@@ -534,8 +592,15 @@ struct Solver {
     reduce_partials(w, nc, 2, sc.ptr + S_RR, cs);
     k_cg_start<<<1, 1, 0, cs>>>(sc.ptr, fl.ptr, rtol, atol, max_it);
     FX_LAUNCH_CHECK("cg_start");
-    auto iteration = [&] {
+    static const int64_t fused_chunks = cgf::capacity(k_cg_fused<T>);  // (thread-safe)
+    const bool fused = nc <= fused_chunks;
+    auto iteration = [&](const PassEnd& end) {
       apply(pp, aa, fl.ptr + F_DONE);
+      if (fused) {
+        cgf::launch(k_cg_fused<T>, nc, cs, sc.ptr, fl.ptr, pp, aa, iv, x, rr, n, lanes, fpart.ptr, meet.ptr, max_it,
+                    end);
+        return;
+      }
       // p.Ap and alpha, then the update, r.r, r.z and beta (each with its levels in the kernel's
       // last block), then p
       if (nc <= kBlockChunks) {
@@ -581,8 +646,9 @@ struct Solver {
         try {
           // kCgPass iterations per pass (every kernel of an iteration skips once the solve is
           // done, so the iterations of a pass after the one that ends the solve are empty)
-          for (int i = 0; i < kCgPass; ++i) iteration();
-          k_cg_cond<<<1, 1, 0, cs>>>(h, fl.ptr, passes.ptr, (max_it + kCgPass - 1) / kCgPass + 2);
+          const int cap = (max_it + kCgPass - 1) / kCgPass + 2;
+          for (int i = 0; i < kCgPass; ++i) iteration(PassEnd{h, passes.ptr, i + 1 < kCgPass ? 0 : cap});
+          if (!fused) k_cg_cond<<<1, 1, 0, cs>>>(h, fl.ptr, passes.ptr, cap);
           FX_LAUNCH_CHECK("cg_condition");
         } catch (...) {
           cudaStreamEndCapture(cs, &body);
@@ -603,6 +669,10 @@ struct Solver {
     FX_CUDA(cudaMemsetAsync(passes.ptr, 0, sizeof(int), cs));
     FX_CUDA(cudaGraphLaunch(G.exec, cs));
     read_state();
+    if (host_flags[F_GAVE_UP]) {
+      FX_CUDA(cudaMemset(meet.ptr, 0, meet.bytes()));
+      throw Error(FX_E_TIMEOUT, "CG: a block did not reach the iteration's reduction");
+    }
     res->converged = host_flags[F_CONV];
     res->iterations = host_flags[F_ITERS];
     res->indefinite = host_flags[F_INDEF];
@@ -1128,6 +1198,9 @@ int fx_solver_create(fx_force* f, int32_t method, fx_solve_opts o, fx_solver** o
       s.passes.alloc(1);
       s.counter.alloc(1);
       FX_CUDA(cudaMemset(s.counter.ptr, 0, sizeof(unsigned)));
+      s.fpart.alloc(static_cast<size_t>(3 * std::max<int64_t>(fx::chunks_of(s.n), 1)));
+      s.meet.alloc(2);
+      FX_CUDA(cudaMemset(s.meet.ptr, 0, s.meet.bytes()));
       s.hbuf.alloc(64);
       s.nres.alloc(n);
       s.ndu.alloc(n);

@@ -29,7 +29,7 @@ extern "C" {
 #define FX_E_NOMEM 3       /* device or host allocation failed */
 #define FX_E_NOT_SPD 4     /* CG met p.Ap <= 0 (SolveResult::indefinite) */
 #define FX_E_DIVERGED 5    /* non-finite values or no convergence */
-#define FX_E_TIMEOUT 6     /* a bounded device wait gave up (reserved: no entry point waits on the device) */
+#define FX_E_TIMEOUT 6     /* a bounded device wait gave up (the fused CG iteration's reductions) */
 #define FX_E_CUDA 7        /* a CUDA runtime error (message in fx_last_error) */
 #define FX_E_UNSTABLE 8    /* an explicit step above the stable step (the stage's io::ModelError) */
 

@@ -1,0 +1,58 @@
+"""The CG iteration in one cooperative launch (cg_fused.cuh) at the edges of its chunks, on a B200: a
+few iterations of ConjugateGradient on distorted bricks (the exact operator) against the same
+recurrence in numpy on the oracle's operator, for vectors of less than one chunk of 2048, just over
+one, odd lengths and many chunks, lane counts 1, 7 and 32, and a solution vector off the pairs'
+16-byte alignment. The two differ by rounding: each of the k iterations forms its products and sums
+with relative errors of a few n eps, so 1e-11 of the largest entry bounds them, and a chunk or an
+entry left out shows at 1e-4 and above. The same solve in one batch and alone, and in batches past
+the fused form's size, has the same bits (test_gpu_nbatch.py)."""
+import numpy as np
+import pytest
+
+import femorax_b200 as fx
+from femorax_b200 import meshes
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("no CUDA device", allow_module_level=True)
+DEV = torch.device("cuda:0")
+
+
+def reference(port, b, diag, k):
+    x, r = np.zeros_like(b), b.copy()
+    z = r / diag
+    p, rz = z.copy(), r @ z
+    for _ in range(k):
+        q = port.apply_operator((1.0, 0.0, 0.0), p)
+        alpha = rz / (p @ q)
+        x, r = x + alpha * p, r - alpha * q
+        z = r / diag
+        new = r @ z
+        p, rz = z + (new / rz) * p, new
+    return x
+
+
+@pytest.mark.parametrize("size", [(1, 1, 1), (7, 9, 8), (8, 9, 8), (12, 11, 13), (23, 22, 21)])
+def test_iterates(size, oracle_mod):
+    spec = meshes.distort(meshes.box_model(*size), 0.15, seed=sum(size))
+    spec.fix_node, spec.fix_dof = spec.fix_node[1:], spec.fix_dof[1:]  # odd numbers of equations
+    mesh = fx.Model(spec).compile().mesh()
+    n = mesh.num_equations
+    force, port = fx.InternalForce(mesh), oracle_mod.PortMesh(mesh)
+    b = np.random.default_rng(1).standard_normal(n)
+    d = torch.zeros(n, dtype=torch.float64, device=DEV)
+    force.operator_diagonal(fx.OperatorCoefficients(), d)
+    for lanes in (1, 7, 32):
+        for k in (1, 4):
+            want = reference(port, b, d.cpu().numpy(), k)
+            s = fx.ConjugateGradient(fx.SolveOptions(relative_tolerance=1e-30, max_iterations=k, lanes=lanes))
+            s.setup(fx.MatrixFreeOperator(force))
+            got = []
+            for off in (0, 1):  # the solution vector aligned to pairs, and not
+                x = torch.zeros(n + off, dtype=torch.float64, device=DEV)[off:]
+                r = s.solve(torch.as_tensor(b, device=DEV), x)
+                assert r.iterations == k and not r.converged
+                got.append(x.cpu().numpy())
+            assert np.max(np.abs(got[0] - want)) <= 1e-11 * np.max(np.abs(want)), (lanes, k)
+            assert np.array_equal(got[0], got[1])
