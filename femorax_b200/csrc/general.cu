@@ -285,22 +285,47 @@ __global__ void __launch_bounds__(kBlock) k_element_force(const double* __restri
   for (int a = 0; a < 24; ++a) slots[static_cast<int64_t>(a) * P + e] = fe[a];
 }
 
-// Soil-material sets (PressureIndependMultiYield: kind 2, PressureDependMultiYield: kind 3), point by
-// point: thread t is point gp = t / P of element e = t % P (consecutive threads, consecutive elements:
-// every state value is read and written as whole lines); stress and compact tangent out. Yielding
-// and failed points counted per warp.
-FX_HD bool soil_point_update(const PimySet& m, const double xl[3][8], const double* ue, int gp, const double* c,
-                             double* t, int64_t stride, double* sg, double* tc, bool* pl) {
-  return point_update_pimy(m, xl, ue, gp, c, t, stride, sg, tc, pl);
-}
-FX_HD bool soil_point_update(const PdmySet& m, const double xl[3][8], const double* ue, int gp, const double* c,
-                             double* t, int64_t stride, double* sg, double* tc, bool* pl) {
-  return point_update_pdmy(m, xl, ue, gp, c, t, stride, sg, tc, pl);
-}
 FX_HD void soil_compact_D(const PimySet&, const double* t, double* D) { pimy::compact_D(t, D); }
 FX_HD void soil_compact_D(const PdmySet& m, const double* t, double* D) { pdmy::compact_D(m.p, t, D); }
+
+FX_HD bool soil_update_strain(const PimySet& m, const double* eps, int gp, const double* c, double* t, int64_t stride,
+                              double* sg, double* tc, bool* pl) {
+  return pimy::update_compact(m.p, m.stage, pimy::Slab<const double>{c + gp * stride, 8 * stride},
+                              pimy::Slab<double>{t + gp * stride, 8 * stride}, eps, sg, tc, pl);
+}
+FX_HD bool soil_update_strain(const PdmySet& m, const double* eps, int gp, const double* c, double* t, int64_t stride,
+                              double* sg, double* tc, bool* pl) {
+  return pdmy::update_compact(m.p, m.stage, pimy::Slab<const double>{c + gp * stride, 8 * stride},
+                              pimy::Slab<double>{t + gp * stride, 8 * stride}, eps, sg, tc, pl);
+}
+
+// Stiffness-proportional damping stress of a point from its strain rate (the reference's
+// point_update_shape, src/physics/elements/std_brick.hpp:419-434, without betaKinit): betaK times this
+// update's tangent, as the material returned it, plus betaKcomm times the committed one.
+template <class Set, int KTAN>
+__device__ void soil_damping(const Set& m, const ParamGP& p, const double* tc, const double* pc, int gp, int64_t P,
+                             const double rate[6], double sd[6]) {
+  double D[36];
+  soil_compact_D(m, tc, D);
+  for (int i = 0; i < 36; ++i) D[i] = p.betaK * D[i];
+  if (p.betaKcomm != 0.0) add_committed_D(m, pc, gp, P, p.betaKcomm, D);
+  for (int a = 0; a < 6; ++a) {
+    double sum = 0.0;
+    for (int c = 0; c < 6; ++c) sum += D[6 * a + c] * rate[c];
+    sd[a] = sum;
+  }
+}
+
+// Soil-material sets (PressureIndependMultiYield: kind 2, PressureDependMultiYield: kind 3), point by
+// point in the layout of points.cuh (warp g point g, lane l element l of the block's 32): every state
+// value is read and written as whole lines, and the element's coordinates and values are staged once
+// for its eight points (a thread per point that gathered them itself held them in local memory, past
+// the L1 cache's size). Stress and compact tangent out; yielding and failed points counted per warp.
+// Bound by the latency of the state's loads and of local memory; B200, with the moved surfaces alone
+// copied: an explicit step of a plastic PressureIndependMultiYield box of 97,336 elements 1.85 -> 0.68
+// ms.
 template <class Set, int KIND, int KTAN, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_soil_points(const double* __restrict__ coords, const int32_t* __restrict__ node,
+__global__ void __launch_bounds__(points::kThreads, MINB) k_soil_points(const double* __restrict__ coords, const int32_t* __restrict__ node,
                                                      const int32_t* __restrict__ eq, const int32_t* __restrict__ param,
                                                      const ParamGP* __restrict__ params, const Set* __restrict__ sets,
                                                      int32_t N, int32_t P, int32_t count, const double* __restrict__ u,
@@ -308,37 +333,31 @@ __global__ void __launch_bounds__(128, MINB) k_soil_points(const double* __restr
                                                      double* __restrict__ ptan, double* __restrict__ psig,
                                                      int* __restrict__ plastic, int* __restrict__ failed,
                                                      const double* __restrict__ v, double* __restrict__ psd) {
-  const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  const int32_t e = static_cast<int32_t>(t % P), gp = static_cast<int32_t>(t / P);
+  __shared__ points::Stage<2, 0> S;
+  points::stage_elements(S, coords, node, eq, N, P, count, u, psd ? v : nullptr);
+  const int gp = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int32_t e = static_cast<int32_t>(blockIdx.x) * points::kEl + l;
   bool pl = false, bad = false;
-  if (gp < 8 && e < count) {
-    const ParamGP p = params[param[e]];
+  if (e < count) {
+    const ParamGP& p = params[param[e]];
     if (p.kind == KIND) {
-      double xl[3][8], ue[24], sg[6], tc[KTAN];
-      load_coords(coords, node, N, P, e, xl);
-      for (int a = 0; a < 24; ++a) {
-        const int32_t q = eq[static_cast<int64_t>(a) * P + e];
-        ue[a] = q >= 0 ? u[q] : 0.0;
-      }
-      bad = !soil_point_update(sets[p.table], xl, ue, gp, pc + e, pt + e, P, sg, tc, &pl);
+      double dN[3][8], dvol, eps[6], sg[6], tc[KTAN], rate[6];
+      const bool damped = psd && (p.betaK != 0.0 || p.betaKcomm != 0.0);
+      points::shape(S, S.tab[gp], l, dN, dvol);
+      points::strain(dN, S.x[0], l, eps);
+      if (damped) points::strain(dN, S.x[1], l, rate);
+      bad = !soil_update_strain(sets[p.table], eps, gp, pc + e, pt + e, P, sg, tc, &pl);
       for (int c = 0; c < 6; ++c) psig[(static_cast<int64_t>(c) * 8 + gp) * P + e] = sg[c];
       for (int c = 0; c < KTAN; ++c) ptan[(static_cast<int64_t>(c) * 8 + gp) * P + e] = tc[c];
-      if (psd && (p.betaK != 0.0 || p.betaKcomm != 0.0)) {  // the damping stress: betaK times this
-        double D[36], ve[24], sd[6];                         // update's tangent + betaKcomm times the
-        soil_compact_D(sets[p.table], tc, D);                // committed one
-        for (int i = 0; i < 36; ++i) D[i] = p.betaK * D[i];
-        if (p.betaKcomm != 0.0) add_committed_D(sets[p.table], pc + e, gp, P, p.betaKcomm, D);
-        for (int a = 0; a < 24; ++a) {
-          const int32_t q = eq[static_cast<int64_t>(a) * P + e];
-          ve[a] = q >= 0 ? v[q] : 0.0;
-        }
-        damping_stress(D, xl, ve, gp, sd);
+      if (damped) {
+        double sd[6];
+        soil_damping<Set, KTAN>(sets[p.table], p, tc, pc + e, gp, P, rate, sd);
         for (int c = 0; c < 6; ++c) psd[(static_cast<int64_t>(c) * 8 + gp) * P + e] = sd[c];
       }
     }
   }
   const unsigned np = __popc(__ballot_sync(0xffffffffu, pl)), nb = __popc(__ballot_sync(0xffffffffu, bad));
-  if ((threadIdx.x & 31) == 0) {
+  if (l == 0) {
     if (np) atomicAdd(plastic, static_cast<int>(np));
     if (nb) atomicAdd(failed, static_cast<int>(nb));
   }
@@ -362,35 +381,8 @@ FX_HD bool soil_predict(const PdmySet& m, const double* eps, int gp, const doubl
   return pdmy::predict_compact(m.p, m.stage, pimy::Slab<const double>{c + gp * stride, 8 * stride},
                                pimy::Slab<double>{t + gp * stride, 8 * stride}, eps, sg, tc, ok);
 }
-FX_HD bool soil_update_strain(const PimySet& m, const double* eps, int gp, const double* c, double* t, int64_t stride,
-                              double* sg, double* tc, bool* pl) {
-  return pimy::update_compact(m.p, m.stage, pimy::Slab<const double>{c + gp * stride, 8 * stride},
-                              pimy::Slab<double>{t + gp * stride, 8 * stride}, eps, sg, tc, pl);
-}
-FX_HD bool soil_update_strain(const PdmySet& m, const double* eps, int gp, const double* c, double* t, int64_t stride,
-                              double* sg, double* tc, bool* pl) {
-  return pdmy::update_compact(m.p, m.stage, pimy::Slab<const double>{c + gp * stride, 8 * stride},
-                              pimy::Slab<double>{t + gp * stride, 8 * stride}, eps, sg, tc, pl);
-}
-
-// The damping stress of a point from its strain rate: betaK times this update's tangent plus betaKcomm
-// times the committed one (damping_stress's sum, the rate already formed).
-template <class Set, int KTAN>
-__device__ void soil_damping(const Set& m, const ParamGP& p, const double* tc, const double* pc, int gp, int64_t P,
-                             const double rate[6], double sd[6]) {
-  double D[36];
-  soil_compact_D(m, tc, D);
-  for (int i = 0; i < 36; ++i) D[i] = p.betaK * D[i];
-  if (p.betaKcomm != 0.0) add_committed_D(m, pc, gp, P, p.betaKcomm, D);
-  for (int a = 0; a < 6; ++a) {
-    double sum = 0.0;
-    for (int c = 0; c < 6; ++c) sum += D[6 * a + c] * rate[c];
-    sd[a] = sum;
-  }
-}
-
 template <class Set, int KIND, int KTAN, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_soil_predict(const double* __restrict__ coords, const int32_t* __restrict__ node,
+__global__ void __launch_bounds__(points::kThreads, MINB) k_soil_predict(const double* __restrict__ coords, const int32_t* __restrict__ node,
                                                       const int32_t* __restrict__ eq, const int32_t* __restrict__ param,
                                                       const ParamGP* __restrict__ params, const Set* __restrict__ sets,
                                                       int32_t N, int32_t P, int32_t count, const double* __restrict__ u,
@@ -399,31 +391,20 @@ __global__ void __launch_bounds__(128, MINB) k_soil_predict(const double* __rest
                                                       int* __restrict__ failed, const double* __restrict__ v,
                                                       double* __restrict__ psd, double* __restrict__ peps,
                                                       double* __restrict__ prate, int* __restrict__ flag) {
-  const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  const int32_t e = static_cast<int32_t>(t % P), gp = static_cast<int32_t>(t / P);
+  __shared__ points::Stage<2, 0> S;
+  points::stage_elements(S, coords, node, eq, N, P, count, u, psd ? v : nullptr);
+  const int gp = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int32_t e = static_cast<int32_t>(blockIdx.x) * points::kEl + l;
   bool bad = false;
-  if (gp < 8) {  // every point of the padded batch gets its flag (padding: 0)
+  if (e < P) {  // every point of the padded batch gets its flag (padding: 0)
     int f = 0;
-    const ParamGP p = params[param[e < count ? e : 0]];
+    const ParamGP& p = params[param[e < count ? e : 0]];
     if (e < count && p.kind == KIND) {
-      double xl[3][8], ue[24], eps[6], sg[6], tc[KTAN], rate[6];
-      load_coords(coords, node, N, P, e, xl);
-      for (int a = 0; a < 24; ++a) {
-        const int32_t q = eq[static_cast<int64_t>(a) * P + e];
-        ue[a] = q >= 0 ? u[q] : 0.0;
-      }
-      PointShape s;
-      point_shape(xl, gp, s);
-      strain_of(s, ue, eps);
+      double dN[3][8], dvol, eps[6], sg[6], tc[KTAN], rate[6];
+      points::shape(S, S.tab[gp], l, dN, dvol);
+      points::strain(dN, S.x[0], l, eps);
       const bool damped = psd && (p.betaK != 0.0 || p.betaKcomm != 0.0);
-      if (damped) {
-        double ve[24];
-        for (int a = 0; a < 24; ++a) {
-          const int32_t q = eq[static_cast<int64_t>(a) * P + e];
-          ve[a] = q >= 0 ? v[q] : 0.0;
-        }
-        strain_of(s, ve, rate);
-      }
+      if (damped) points::strain(dN, S.x[1], l, rate);
       bool ok = true;
       if (soil_predict(sets[p.table], eps, gp, pc + e, pt + e, P, sg, tc, &ok)) {
         f = 1;
@@ -441,10 +422,10 @@ __global__ void __launch_bounds__(128, MINB) k_soil_predict(const double* __rest
         }
       }
     }
-    flag[t] = f;
+    flag[static_cast<int64_t>(gp) * P + e] = f;
   }
   const unsigned nb = __popc(__ballot_sync(0xffffffffu, bad));
-  if ((threadIdx.x & 31) == 0 && nb) atomicAdd(failed, static_cast<int>(nb));
+  if (l == 0 && nb) atomicAdd(failed, static_cast<int>(nb));
 }
 
 constexpr int kScanBlock = 256;
@@ -554,7 +535,8 @@ __global__ void __launch_bounds__(kBlock) k_soil_force(const double* __restrict_
 }
 
 // commitState of the PressureIndependMultiYield points: the scalar values of every point, the
-// surfaces of the points whose last update changed them (the others' committed surfaces stand).
+// surfaces that their last update changed (value S_CHANGED: 1 every surface, else a bit per moved
+// center; the others' committed surfaces stand).
 __global__ void __launch_bounds__(256) k_pimy_commit(const int32_t* __restrict__ param,
                                                      const ParamGP* __restrict__ params,
                                                      const PimySet* __restrict__ pimy, int32_t P, int32_t count,
@@ -565,10 +547,21 @@ __global__ void __launch_bounds__(256) k_pimy_commit(const int32_t* __restrict__
   const ParamGP& p = params[param[e]];
   if (p.kind != 2) return;
   const int64_t base = static_cast<int64_t>(gp) * P + e, ld = 8 * static_cast<int64_t>(P);
-  for (int k = 0; k < pimy::S_SURF; ++k) pc[base + k * ld] = pt[base + k * ld];
-  if (pt[base + pimy::S_CHANGED * ld] != 0.0) {
-    const int n = pimy::nstate(pimy[p.table].p.ns);
-    for (int k = pimy::S_SURF; k < n; ++k) pc[base + k * ld] = pt[base + k * ld];
+  const pimy::Slab<const double> T{pt + base, ld};
+  const pimy::Slab<double> C{pc + base, ld};
+  const double changed = T[pimy::S_CHANGED];
+  pimy::copy_values(T, C, 0, pimy::S_SURF);
+  if (changed == 1.0) {
+    pimy::copy_values(T, C, pimy::S_SURF, pimy::nstate(pimy[p.table].p.ns));
+  } else {
+    for (uint64_t moved = static_cast<uint64_t>(changed); moved; moved &= moved - 1) {
+      const int k = pimy::S_SURF + 8 * (__ffsll(static_cast<long long>(moved)) - 2) + 2;  // surface i: bit i
+      double c[6];
+#pragma unroll
+      for (int i = 0; i < 6; ++i) c[i] = T[k + i];
+#pragma unroll
+      for (int i = 0; i < 6; ++i) C[k + i] = c[i];
+    }
   }
 }
 
@@ -1139,31 +1132,34 @@ void general_diagonal(ForceState& s, const double k[3], double* d, cudaStream_t 
   FX_LAUNCH_CHECK("slot_gather");
 }
 
+// Blocks of 256 points per SM the soil point kernels' registers are sized for (80 and 128 per thread)
+constexpr int kPimyBlocks = 3, kPdmyBlocks = 2;
+
 // The compacted corrector's passes for the points of one soil kind (the per-point buffers allocated
 // at the first call: strain and strain rate, 48 bytes per point each, a flag and a list entry).
-template <class Set, int KIND, int KTAN, int MINB>
+template <class Set, int KIND, int KTAN, int MINB, int MINC>
 void soil_points_compacted(ForceState& s, const Set* sets, const double* u, const double* v, const double* pc,
                            double* pt, double* ptan, double* psig, cudaStream_t st) {
-  const int64_t points = static_cast<int64_t>(8) * s.P;
-  const unsigned nb = static_cast<unsigned>((points + kScanBlock - 1) / kScanBlock);
-  if (s.soil_eps.n < static_cast<size_t>(6 * points)) {
-    s.soil_eps.alloc(static_cast<size_t>(6 * points));
-    if (s.soil_sd.n) s.soil_rate.alloc(static_cast<size_t>(6 * points));
-    s.soil_flag.alloc(static_cast<size_t>(points));
-    s.soil_list.alloc(static_cast<size_t>(points));
+  const int64_t points_n = static_cast<int64_t>(8) * s.P;
+  const unsigned nb = static_cast<unsigned>((points_n + kScanBlock - 1) / kScanBlock);
+  if (s.soil_eps.n < static_cast<size_t>(6 * points_n)) {
+    s.soil_eps.alloc(static_cast<size_t>(6 * points_n));
+    if (s.soil_sd.n) s.soil_rate.alloc(static_cast<size_t>(6 * points_n));
+    s.soil_flag.alloc(static_cast<size_t>(points_n));
+    s.soil_list.alloc(static_cast<size_t>(points_n));
     s.soil_counts.alloc(nb);
     s.soil_total.alloc(1);
   }
-  k_soil_predict<Set, KIND, KTAN, MINB><<<static_cast<unsigned>((points + 127) / 128), 128, 0, st>>>(
+  k_soil_predict<Set, KIND, KTAN, MINB><<<grid_for(s.P, points::kEl), points::kThreads, 0, st>>>(
       s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr, s.params.ptr, sets, s.N, s.P, s.count, u, pc, pt, ptan, psig,
       s.pimy_failed.ptr, v, s.soil_sd.ptr, s.soil_eps.ptr, s.soil_rate.ptr, s.soil_flag.ptr);
   FX_LAUNCH_CHECK("soil_predict");
-  k_flag_counts<<<nb, kScanBlock, 0, st>>>(s.soil_flag.ptr, points, s.soil_counts.ptr);
+  k_flag_counts<<<nb, kScanBlock, 0, st>>>(s.soil_flag.ptr, points_n, s.soil_counts.ptr);
   k_flag_offsets<<<1, 1024, 0, st>>>(s.soil_counts.ptr, static_cast<int>(nb), s.soil_total.ptr);
-  k_flag_list<<<nb, kScanBlock, 0, st>>>(s.soil_flag.ptr, points, s.soil_counts.ptr, s.soil_list.ptr);
+  k_flag_list<<<nb, kScanBlock, 0, st>>>(s.soil_flag.ptr, points_n, s.soil_counts.ptr, s.soil_list.ptr);
   FX_LAUNCH_CHECK("soil_compaction");
-  const unsigned cg = static_cast<unsigned>(std::min<int64_t>((points + 127) / 128, static_cast<int64_t>(num_sms()) * 8));
-  k_soil_correct<Set, KIND, KTAN, MINB><<<cg, 128, 0, st>>>(s.param.ptr, s.params.ptr, sets, s.P, s.soil_list.ptr,
+  const unsigned cg = static_cast<unsigned>(std::min<int64_t>((points_n + 127) / 128, static_cast<int64_t>(num_sms()) * 8));
+  k_soil_correct<Set, KIND, KTAN, MINC><<<cg, 128, 0, st>>>(s.param.ptr, s.params.ptr, sets, s.P, s.soil_list.ptr,
                                                              s.soil_total.ptr, pc, pt, ptan, psig, s.plastic_dev.ptr,
                                                              s.pimy_failed.ptr, s.soil_eps.ptr, s.soil_rate.ptr,
                                                              s.soil_sd.ptr);
@@ -1179,16 +1175,15 @@ void general_force(ForceState& s, const double* u, const double* v, double* f, c
                                                                    s.j2_committed.ptr, s.j2_trial.ptr, s.j2_tan.ptr,
                                                                    s.plastic_dev.ptr, s.ssp_geo.ptr, s.ssp_con.ptr);
   FX_LAUNCH_CHECK("element_force");
-  const int64_t points = static_cast<int64_t>(8) * s.P;
   if (s.has_pimy && s.count > 0 && s.compact_soil) {
-    soil_points_compacted<PimySet, 2, pimy::kTan, 6>(s, s.pimy_dev.ptr, u, v, s.pimy_committed.ptr, s.pimy_trial.ptr,
+    soil_points_compacted<PimySet, 2, pimy::kTan, kPimyBlocks, 6>(s, s.pimy_dev.ptr, u, v, s.pimy_committed.ptr, s.pimy_trial.ptr,
                                                       s.pimy_tan.ptr, s.pimy_sig.ptr, st);
     k_soil_force<<<grid_for(s.count, kBlock), kBlock, 0, st>>>(s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr,
                                                                s.params.ptr, s.N, s.P, s.count, v, s.pimy_sig.ptr,
                                                                s.soil_sd.ptr, s.slots.ptr, 2);
     FX_LAUNCH_CHECK("pimy_force");
   } else if (s.has_pimy && s.count > 0) {
-    k_soil_points<PimySet, 2, pimy::kTan, 6><<<static_cast<unsigned>((points + 127) / 128), 128, 0, st>>>(
+    k_soil_points<PimySet, 2, pimy::kTan, kPimyBlocks><<<grid_for(s.count, points::kEl), points::kThreads, 0, st>>>(
         s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr, s.params.ptr, s.pimy_dev.ptr, s.N, s.P, s.count, u,
         s.pimy_committed.ptr, s.pimy_trial.ptr, s.pimy_tan.ptr, s.pimy_sig.ptr, s.plastic_dev.ptr, s.pimy_failed.ptr,
         v, s.soil_sd.ptr);
@@ -1199,14 +1194,14 @@ void general_force(ForceState& s, const double* u, const double* v, double* f, c
     FX_LAUNCH_CHECK("pimy_force");
   }
   if (s.has_pdmy && s.count > 0 && s.compact_soil) {
-    soil_points_compacted<PdmySet, 3, pdmy::kTan, 4>(s, s.pdmy_dev.ptr, u, v, s.pdmy_committed.ptr, s.pdmy_trial.ptr,
+    soil_points_compacted<PdmySet, 3, pdmy::kTan, kPdmyBlocks, 4>(s, s.pdmy_dev.ptr, u, v, s.pdmy_committed.ptr, s.pdmy_trial.ptr,
                                                       s.pdmy_tan.ptr, s.pdmy_sig.ptr, st);
     k_soil_force<<<grid_for(s.count, kBlock), kBlock, 0, st>>>(s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr,
                                                                s.params.ptr, s.N, s.P, s.count, v, s.pdmy_sig.ptr,
                                                                s.soil_sd.ptr, s.slots.ptr, 3);
     FX_LAUNCH_CHECK("pdmy_force");
   } else if (s.has_pdmy && s.count > 0) {
-    k_soil_points<PdmySet, 3, pdmy::kTan, 4><<<static_cast<unsigned>((points + 127) / 128), 128, 0, st>>>(
+    k_soil_points<PdmySet, 3, pdmy::kTan, kPdmyBlocks><<<grid_for(s.count, points::kEl), points::kThreads, 0, st>>>(
         s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr, s.params.ptr, s.pdmy_dev.ptr, s.N, s.P, s.count, u,
         s.pdmy_committed.ptr, s.pdmy_trial.ptr, s.pdmy_tan.ptr, s.pdmy_sig.ptr, s.plastic_dev.ptr, s.pimy_failed.ptr,
         v, s.soil_sd.ptr);

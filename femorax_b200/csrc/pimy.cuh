@@ -156,6 +156,26 @@ struct Slab {
   FX_PIMY_HD T& operator[](int k) const { return p[k * ld]; }
 };
 
+// T[k] = C[k] for k in [k0, k1), 16 values read ahead of their stores: one value at a time the copy is
+// a chain of memory latencies.
+template <class CV, class TV>
+FX_PIMY_HD inline void copy_values(const CV& C, const TV& T, int k0, int k1) {
+  constexpr int B = 16;
+  int k = k0;
+  for (; k + B <= k1; k += B) {
+    double v[B];
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int i = 0; i < B; ++i) v[i] = C[k + i];
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int i = 0; i < B; ++i) T[k + i] = v[i];
+  }
+  for (; k < k1; ++k) T[k] = C[k];
+}
+
 // MultiYieldSurface's secondOrderEqn: the smaller non-negative root of A x^2 + B x + C; `ok` false
 // (and NaN) where OpenSees stops the program.
 FX_PIMY_HD inline double quad_root(double A, double B, double C, bool& ok) {
@@ -350,9 +370,10 @@ FX_PIMY_HD inline int to_int(double x) {  // C++ truncation, NaN 0 and clamped o
 
 // One point's update from its committed state C to the trial state T at the total strain eps
 // (engineering shear): OpenSees' setTrialStrain + getStress + getTangent, the instance's members as
-// locals. The surfaces are read from the committed state until the update first changes one; then
-// all of them are copied to the trial state, which holds them from there on (copy on write: most
-// updates change no surface). `full`: the trial state's surfaces are written in any case.
+// locals. A surface's center is read from the committed state until the update changes it; from there
+// on the trial state holds it (`moved`, bit i for surface i: most updates move one surface or none).
+// Sizes and plastic moduli change at the switch to the plastic stage only, where the trial state takes
+// every surface (`scaled`). `full`: the trial state's surfaces are written in any case.
 template <class CV, class TV>
 struct Point {
   const Params& P;
@@ -360,7 +381,8 @@ struct Point {
   CV C;
   TV T;
   bool full = true;
-  bool dirty = false;  // the trial state holds the surfaces
+  bool scaled = false;
+  uint64_t moved = 0;
   bool ok = true;  // false after a state OpenSees stops the program for
   Ten cur, strain, trial, rate, sub;  // currentStress, currentStrain, trialStress, strainRate, subStrainRate
   int active_c = 0, active = 0, e2p = 0;
@@ -369,20 +391,15 @@ struct Point {
   FX_PIMY_HD Point(const Params& p, int st, CV c, TV t) : P(p), stage(st), C(c), T(t) {}
 
   FX_PIMY_HD int at(int i) const { return S_SURF + 8 * (i - 1); }
-  FX_PIMY_HD double sv(int k) const { return dirty ? T[k] : C[k]; }
-  FX_PIMY_HD void touch() {  // the first change: the surfaces into the trial state
-    if (dirty) return;
-    for (int k = S_SURF; k < nstate(P.ns); ++k) T[k] = C[k];
-    dirty = true;
-  }
-  FX_PIMY_HD double size(int i) const { return i == 0 ? 0. : sv(at(i)); }
-  FX_PIMY_HD double hmod(int i) const { return i == 0 ? 0. : sv(at(i) + 1); }
+  FX_PIMY_HD double size(int i) const { return i == 0 ? 0. : scaled ? T[at(i)] : C[at(i)]; }
+  FX_PIMY_HD double hmod(int i) const { return i == 0 ? 0. : scaled ? T[at(i) + 1] : C[at(i) + 1]; }
   FX_PIMY_HD void center(int i, double* c) const {
-    for (int k = 0; k < 6; ++k) c[k] = i == 0 ? 0. : sv(at(i) + 2 + k);
+    const bool mine = (moved >> i) & 1u;
+    for (int k = 0; k < 6; ++k) c[k] = i == 0 ? 0. : mine ? T[at(i) + 2 + k] : C[at(i) + 2 + k];
   }
   FX_PIMY_HD void set_center(int i, const double* c) {
-    touch();
     for (int k = 0; k < 6; ++k) T[at(i) + 2 + k] = c[k];
+    moved |= uint64_t(1) << i;
   }
 
   FX_PIMY_HD double yield(const Ten& s, int i) const {  // yieldFunc
@@ -445,7 +462,6 @@ struct Point {
     f = pow(f, P.n_press);
     G *= f;
     K *= f;
-    touch();
     for (int i = 1; i <= P.ns; ++i) {
       const double hm = hmod(i) * f, sz = size(i) * h;
       T[at(i)] = sz;
@@ -453,6 +469,7 @@ struct Point {
       const double zero[6] = {0., 0., 0., 0., 0., 0.};
       set_center(i, zero);
     }
+    scaled = true;
   }
 
   FX_PIMY_HD void elastic_to_plastic() {  // elast2Plast
@@ -722,14 +739,15 @@ struct Point {
     T[S_G] = G;
     T[S_K] = K;
     T[S_ACTIVE] = stage == 1 ? active : active_c;
-    if (full) touch();
-    T[S_CHANGED] = dirty ? 1.0 : 0.0;
+    // what a commit copies: 1 every surface, else bit i the center of surface i (exact: ns <= 40)
+    T[S_CHANGED] = full || scaled ? 1.0 : static_cast<double>(moved);
   }
 };
 
 // The update of one point: trial state, stress and tangent (D[6 i + j]) at total strain eps.
 template <class CV, class TV>
 FX_PIMY_HD inline bool update(const Params& p, int stage, CV C, TV T, const double* eps, double* sig, double* D) {
+  copy_values(C, T, S_SURF, nstate(p.ns));
   Point<CV, TV> pt(p, stage, C, T);
   pt.run(eps);
   pt.finish(sig, D);
@@ -737,8 +755,8 @@ FX_PIMY_HD inline bool update(const Params& p, int stage, CV C, TV T, const doub
 }
 
 // The same with the tangent in compact form t[kTan]; *plastic: an active yield surface. Copy on
-// write: the trial state's surfaces are written only if the update changed them (value S_CHANGED),
-// so a commit copies the surfaces of those points only.
+// write: the trial state's surfaces are written only where the update changed them (value S_CHANGED),
+// so a commit copies those only.
 template <class CV, class TV>
 FX_PIMY_HD inline bool update_compact(const Params& p, int stage, CV C, TV T, const double* eps, double* sig, double* t,
                                  bool* plastic) {

@@ -23,32 +23,6 @@ struct PdmySet {
   int stage;
 };
 
-// The update of point gp of element e (the reference's point_update_shape without stiffness
-// damping): strain at the point from the element's displacements, the material update from the
-// committed state to the trial one; the stress and the compact tangent out. Returns the update's ok.
-FX_HD bool point_update_pimy(const PimySet& m, const double xl[3][8], const double* ue, int gp,
-                             const double* committed, double* trial, int64_t stride, double sg[6],
-                             double t[pimy::kTan], bool* plastic) {
-  PointShape s;
-  point_shape(xl, gp, s);
-  double e[6];
-  strain_of(s, ue, e);
-  return pimy::update_compact(m.p, m.stage, pimy::Slab<const double>{committed + gp * stride, 8 * stride},
-                              pimy::Slab<double>{trial + gp * stride, 8 * stride}, e, sg, t, plastic);
-}
-
-// The same for a PressureDependMultiYield point (its trial state written in full).
-FX_HD bool point_update_pdmy(const PdmySet& m, const double xl[3][8], const double* ue, int gp,
-                             const double* committed, double* trial, int64_t stride, double sg[6],
-                             double t[pdmy::kTan], bool* plastic) {
-  PointShape s;
-  point_shape(xl, gp, s);
-  double e[6];
-  strain_of(s, ue, e);
-  return pdmy::update_compact(m.p, m.stage, pimy::Slab<const double>{committed + gp * stride, 8 * stride},
-                              pimy::Slab<double>{trial + gp * stride, 8 * stride}, e, sg, t, plastic);
-}
-
 // Out of line on the device: only betaKcomm sets form the committed tangent, and inlined it would take
 // registers from the common path of the kernels that call it.
 #if defined(__CUDACC__)
@@ -72,23 +46,6 @@ FX_HD_COLD void add_committed_D(const PdmySet& m, const double* committed, int g
   pdmy::committed_compact(m.p, m.stage, pimy::Slab<const double>{committed + gp * stride, 8 * stride}, t);
   pdmy::compact_D(m.p, t, Dc);
   for (int i = 0; i < 36; ++i) M[i] += f * Dc[i];
-}
-
-// Stiffness-proportional damping stress of a point (the reference's point_update_shape,
-// src/physics/elements/std_brick.hpp:419-434, without betaKinit): sd[a] = sum_c Dd[a][c] rate[c],
-// Dd = betaK D (+ betaKcomm Dc when betaKcomm is not zero: add_committed_D), D the point's tangent of
-// this update (as the material returned it, before any mirroring), Dc its committed tangent, rate
-// the strain of the element velocities at the point.
-FX_HD void damping_stress(const double* Dd, const double xl[3][8], const double* ve, int gp, double sd[6]) {
-  PointShape s;
-  point_shape(xl, gp, s);
-  double rate[6];
-  strain_of(s, ve, rate);
-  for (int a = 0; a < 6; ++a) {
-    double sum = 0.0;
-    for (int c = 0; c < 6; ++c) sum += Dd[6 * a + c] * rate[c];
-    sd[a] = sum;
-  }
 }
 
 // Internal force of one element from its points' stresses (point gp's component c at

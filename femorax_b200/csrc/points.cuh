@@ -53,6 +53,17 @@ struct Stage {
   double x[NX][24][kEl];
   double part[8][NP][24][kEl];
   PointTable tab[8];
+  // corner coordinates on their way to the edges (row 3 a + d)
+  __device__ double (*corners())[kEl] { return part[0][0]; }
+};
+// The same for kernels that sum nothing over the points.
+template <int NX>
+struct Stage<NX, 0> {
+  double edge[kEdges][kEl];
+  double x[NX][24][kEl];
+  double xl[24][kEl];
+  PointTable tab[8];
+  __device__ double (*corners())[kEl] { return xl; }
 };
 
 // The block's elements: their edge vectors and their values of x0 (and x1), by all threads; the point
@@ -68,15 +79,15 @@ __device__ __forceinline__ void stage_elements(Stage<NX, NP>& S, const double* _
   int32_t q[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) q[k] = ok ? eq[static_cast<int64_t>(w + 8 * k) * P + e] : -1;
-  // corner w's coordinates pass through the first rows of the points' partial sums
-  double(*xl)[kEl] = &S.part[0][0][0];
+  double(*xl)[kEl] = S.corners();
   const int32_t n = ok ? node[static_cast<int64_t>(w) * P + e] : 0;
 #pragma unroll
   for (int d = 0; d < 3; ++d) xl[3 * w + d][l] = ok ? coords[static_cast<int64_t>(d) * N + n] : 0.0;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     S.x[0][w + 8 * k][l] = q[k] >= 0 ? x0[q[k]] : 0.0;
-    if constexpr (NX == 2) S.x[1][w + 8 * k][l] = q[k] >= 0 ? x1[q[k]] : 0.0;
+    if constexpr (NX == 2)
+      if (x1) S.x[1][w + 8 * k][l] = q[k] >= 0 ? x1[q[k]] : 0.0;
   }
   if (l == 0) point_table(w, S.tab[w]);
   __syncthreads();
