@@ -187,6 +187,7 @@ struct ForceState {
   DeviceArray<int8_t> eq_dof;
   bool has_nodal_mass = false, has_nodal_alpha = false;
   bool any_alpha = false;  // a parameter set with mass-proportional damping
+  bool all_soil = false;   // every parameter set bound to a multi-yield soil
   int path = FX_PATH_AUTO;  // requested
   BoxPlan box;
   // work vectors (host-buffer apply, solvers)

@@ -534,6 +534,73 @@ __global__ void __launch_bounds__(kBlock) k_soil_force(const double* __restrict_
   for (int a = 0; a < 24; ++a) slots[static_cast<int64_t>(a) * P + e] = fe[a];
 }
 
+// The same, point-parallel (points.cuh), where no set carries damping: element_force_from_stress's sums
+// in its order, per point the stress term and then minus the body force, which the sum forms from the
+// point's volume. 64,000 elements, B200: 43 -> 24 us (a thread per element held 255 registers).
+__global__ void __launch_bounds__(points::kThreads, 2)
+    k_soil_force_points(const double* __restrict__ coords, const int32_t* __restrict__ node,
+                        const int32_t* __restrict__ eq, const int32_t* __restrict__ param,
+                        const ParamGP* __restrict__ params, int32_t N, int32_t P, int32_t count,
+                        const double* __restrict__ v, const double* __restrict__ psig, double* __restrict__ slots,
+                        int kind) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  auto& S = *reinterpret_cast<points::Stage<1, 1>*>(raw);
+  __shared__ double vol[8][points::kEl];
+  points::stage_elements(S, coords, node, eq, N, P, count, v, nullptr);
+  const int gp = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int32_t e = static_cast<int32_t>(blockIdx.x) * points::kEl + l;
+  const bool ok = e < count && params[param[e]].kind == kind;
+  if (ok) {
+    double dN[3][8], dvol, sg[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) sg[c] = psig[(static_cast<int64_t>(c) * 8 + gp) * P + e];
+    points::shape(S, S.tab[gp], l, dN, dvol);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) sg[c] = sg[c] * dvol;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      double r[3];
+      points::corner_force(dN, sg, j, r);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) S.part[gp][0][3 * j + q][l] = r[q];
+    }
+    vol[gp][l] = dvol;
+  }
+  __syncthreads();
+  if (!ok) return;
+  const ParamGP& p = params[param[e]];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int a = gp + 8 * k, j = a / 3;
+    const double b = p.b[a % 3];
+    double resid = 0.0;
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      resid += S.part[g][0][a][l];
+      resid -= vol[g][l] * b * S.tab[g].N[j];
+    }
+    slots[static_cast<int64_t>(a) * P + e] = resid + 0.0;
+  }
+}
+
+void soil_force(ForceState& s, const double* v, const double* sig, int kind, cudaStream_t st) {
+  if (!s.any_alpha && !s.soil_sd.ptr) {
+    constexpr int bytes = static_cast<int>(sizeof(points::Stage<1, 1>));
+    static const bool once = [] {  // (thread-safe)
+      FX_CUDA(cudaFuncSetAttribute(k_soil_force_points, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+      return true;
+    }();
+    (void)once;
+    k_soil_force_points<<<grid_for(s.count, points::kEl), points::kThreads, bytes, st>>>(
+        s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr, s.params.ptr, s.N, s.P, s.count, v, sig, s.slots.ptr, kind);
+  } else {
+    k_soil_force<<<grid_for(s.count, kBlock), kBlock, 0, st>>>(s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr,
+                                                               s.params.ptr, s.N, s.P, s.count, v, sig, s.soil_sd.ptr,
+                                                               s.slots.ptr, kind);
+  }
+  FX_LAUNCH_CHECK("soil_force");
+}
+
 // commitState of the PressureIndependMultiYield points: the scalar values of every point, the
 // surfaces that their last update changed (value S_CHANGED: 1 every surface, else a bit per moved
 // center; the others' committed surfaces stand).
@@ -1169,7 +1236,7 @@ void soil_points_compacted(ForceState& s, const Set* sets, const double* u, cons
 void general_force(ForceState& s, const double* u, const double* v, double* f, cudaStream_t st) {
   if (general_fast_applies(s)) return general_force_fast(s, u, v, f, st);
   if (s.has_j2 || s.has_pimy || s.has_pdmy) FX_CUDA(cudaMemsetAsync(s.plastic_dev.ptr, 0, sizeof(int), st));
-  if (s.count > 0)
+  if (s.count > 0 && !s.all_soil)
     k_element_force<<<grid_for(s.count, kBlock), kBlock, 0, st>>>(s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr,
                                                                    s.params.ptr, s.N, s.P, s.count, u, v, s.slots.ptr,
                                                                    s.j2_committed.ptr, s.j2_trial.ptr, s.j2_tan.ptr,
@@ -1178,38 +1245,26 @@ void general_force(ForceState& s, const double* u, const double* v, double* f, c
   if (s.has_pimy && s.count > 0 && s.compact_soil) {
     soil_points_compacted<PimySet, 2, pimy::kTan, kPimyBlocks, 6>(s, s.pimy_dev.ptr, u, v, s.pimy_committed.ptr, s.pimy_trial.ptr,
                                                       s.pimy_tan.ptr, s.pimy_sig.ptr, st);
-    k_soil_force<<<grid_for(s.count, kBlock), kBlock, 0, st>>>(s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr,
-                                                               s.params.ptr, s.N, s.P, s.count, v, s.pimy_sig.ptr,
-                                                               s.soil_sd.ptr, s.slots.ptr, 2);
-    FX_LAUNCH_CHECK("pimy_force");
+    soil_force(s, v, s.pimy_sig.ptr, 2, st);
   } else if (s.has_pimy && s.count > 0) {
     k_soil_points<PimySet, 2, pimy::kTan, kPimyBlocks><<<grid_for(s.count, points::kEl), points::kThreads, 0, st>>>(
         s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr, s.params.ptr, s.pimy_dev.ptr, s.N, s.P, s.count, u,
         s.pimy_committed.ptr, s.pimy_trial.ptr, s.pimy_tan.ptr, s.pimy_sig.ptr, s.plastic_dev.ptr, s.pimy_failed.ptr,
         v, s.soil_sd.ptr);
     FX_LAUNCH_CHECK("pimy_points");
-    k_soil_force<<<grid_for(s.count, kBlock), kBlock, 0, st>>>(s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr,
-                                                               s.params.ptr, s.N, s.P, s.count, v, s.pimy_sig.ptr,
-                                                               s.soil_sd.ptr, s.slots.ptr, 2);
-    FX_LAUNCH_CHECK("pimy_force");
+    soil_force(s, v, s.pimy_sig.ptr, 2, st);
   }
   if (s.has_pdmy && s.count > 0 && s.compact_soil) {
     soil_points_compacted<PdmySet, 3, pdmy::kTan, kPdmyBlocks, 4>(s, s.pdmy_dev.ptr, u, v, s.pdmy_committed.ptr, s.pdmy_trial.ptr,
                                                       s.pdmy_tan.ptr, s.pdmy_sig.ptr, st);
-    k_soil_force<<<grid_for(s.count, kBlock), kBlock, 0, st>>>(s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr,
-                                                               s.params.ptr, s.N, s.P, s.count, v, s.pdmy_sig.ptr,
-                                                               s.soil_sd.ptr, s.slots.ptr, 3);
-    FX_LAUNCH_CHECK("pdmy_force");
+    soil_force(s, v, s.pdmy_sig.ptr, 3, st);
   } else if (s.has_pdmy && s.count > 0) {
     k_soil_points<PdmySet, 3, pdmy::kTan, kPdmyBlocks><<<grid_for(s.count, points::kEl), points::kThreads, 0, st>>>(
         s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr, s.params.ptr, s.pdmy_dev.ptr, s.N, s.P, s.count, u,
         s.pdmy_committed.ptr, s.pdmy_trial.ptr, s.pdmy_tan.ptr, s.pdmy_sig.ptr, s.plastic_dev.ptr, s.pimy_failed.ptr,
         v, s.soil_sd.ptr);
     FX_LAUNCH_CHECK("pdmy_points");
-    k_soil_force<<<grid_for(s.count, kBlock), kBlock, 0, st>>>(s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr,
-                                                               s.params.ptr, s.N, s.P, s.count, v, s.pdmy_sig.ptr,
-                                                               s.soil_sd.ptr, s.slots.ptr, 3);
-    FX_LAUNCH_CHECK("pdmy_force");
+    soil_force(s, v, s.pdmy_sig.ptr, 3, st);
   }
   const double* m2 = s.has_nodal_alpha ? s.nodal_alpha_mass.ptr : nullptr;
   if (s.neq > 0)

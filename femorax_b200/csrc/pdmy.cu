@@ -205,6 +205,8 @@ int fx_force_set_pdmy(fx_force* f, int32_t set, const fx_pdmy* m) {
       s.pdmy_h[q.table] = fx::PdmySet{m->p, 0};
     }
     q.kind = 3;
+    s.all_soil = true;
+    for (const auto& each : s.params_h) s.all_soil = s.all_soil && each.kind >= 2;
     FX_CUDA(cudaMemcpy(s.pdmy_dev.ptr, s.pdmy_h.data(), sizeof(fx::PdmySet) * s.pdmy_h.size(), cudaMemcpyHostToDevice));
     FX_CUDA(cudaMemcpy(s.params.ptr, s.params_h.data(), sizeof(fx::ParamGP) * s.params_h.size(), cudaMemcpyHostToDevice));
     s.has_pdmy = true;

