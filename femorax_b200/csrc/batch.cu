@@ -255,7 +255,8 @@ __global__ void k_b_inner_start(double* sc, int* fl, const int* used, int nslots
   f[F_DONE] = f[F_CONV] || f[F_MAXIT] <= 0;
 }
 
-// The inner CG's vector kernels in two forms with the same arithmetic and sums: BLOCK, a block of
+// The inner CG's vector kernels for batches past the fused launch's size (below), in two forms
+// with the same arithmetic and sums: BLOCK, a block of
 // kChunkBlock threads per chunk (every entry's loads in flight at once, the chunk's sums by one warp
 // from shared memory), for batches of at most kBlockChunks chunks; otherwise a warp per chunk (8 per
 // block, lane_loop). Both launch 256 threads per block.

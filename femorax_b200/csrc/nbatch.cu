@@ -225,7 +225,8 @@ __global__ void k_nb_cg_start(double* sc, int* fl, int count, double rtol, doubl
   f[G_CG_DONE] = f[G_CG_CONV] || max_it <= 0;
 }
 
-// The CG's vector kernels in two forms with the same arithmetic and sums: BLOCK, a block of
+// The CG's vector kernels for batches past the fused launch's size (below), in two forms
+// with the same arithmetic and sums: BLOCK, a block of
 // kChunkBlock threads per chunk (every entry's loads in flight at once, the chunk's sums by one warp
 // from shared memory), for combined meshes of at most kBlockChunks chunks; otherwise a warp per
 // chunk (8 per block, lane_loop). Both launch 256 threads per block.
