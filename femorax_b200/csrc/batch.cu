@@ -1001,6 +1001,8 @@ int fx_engine_create(int32_t device, int64_t capacity, int32_t max_slots, fx_coe
       FX_CUDA(cudaMemcpy(e.fl.ptr, f0.data(), sizeof(int) * f0.size(), cudaMemcpyHostToDevice));
       FX_CUDA(cudaMemset(e.sc.ptr, 0, sizeof(double) * fx::NSC * max_slots));
       FX_CUDA(cudaMemset(e.used_dev.ptr, 0, sizeof(int) * max_slots));
+      // these are on the legacy stream; the engine's own does not wait for it
+      FX_CUDA(cudaStreamSynchronize(nullptr));
     } catch (...) {
       delete h;
       throw;

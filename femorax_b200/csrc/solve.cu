@@ -1219,6 +1219,9 @@ int fx_solver_create(fx_force* f, int32_t method, fx_solve_opts o, fx_solver** o
         s.ap32.alloc(n);
         s.d32.alloc(n);
       }
+      // the counters' zeros are on the legacy stream; the solves run on the solver's own, which does not
+      // wait for it
+      FX_CUDA(cudaStreamSynchronize(nullptr));
     } catch (...) {
       delete h;
       throw;

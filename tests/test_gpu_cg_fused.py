@@ -56,3 +56,38 @@ def test_iterates(size, oracle_mod):
                 got.append(x.cpu().numpy())
             assert np.max(np.abs(got[0] - want)) <= 1e-11 * np.max(np.abs(want)), (lanes, k)
             assert np.array_equal(got[0], got[1])
+
+
+def test_created_beside_a_busy_default_stream():
+    """A solver's counters start at zero for its own stream's solves also while the default stream, on
+    which they are zeroed, still works through other kernels (and the memory held another solver's
+    counts): creation waits for the zeros. The same solve as with the default stream idle."""
+    def problem(size):
+        spec = meshes.distort(meshes.box_model(*size), 0.15, seed=sum(size))
+        return fx.InternalForce(fx.Model(spec).compile().mesh())
+
+    def solve(force, stream):
+        n = force.num_equations
+        with torch.cuda.stream(stream):
+            b = torch.as_tensor(np.random.default_rng(2).standard_normal(n), device=DEV)
+            x = torch.zeros(n, dtype=torch.float64, device=DEV)
+        stream.synchronize()
+        for _ in range(100):  # (some 50 ms)
+            torch.mm(m, m, out=out)
+        s = fx.ConjugateGradient(fx.SolveOptions(relative_tolerance=1e-30, max_iterations=6))
+        s.setup(fx.MatrixFreeOperator(force), stream=stream)
+        r = s.solve(b, x, stream=stream)
+        stream.synchronize()
+        torch.cuda.synchronize()
+        return r, x.cpu().numpy()
+
+    small, large = problem((8, 9, 8)), problem((12, 11, 13))
+    m = torch.randn(2048, 2048, dtype=torch.float64, device=DEV)
+    out = torch.empty_like(m)
+    side = torch.cuda.Stream()
+    idle_r, idle = solve(small, torch.cuda.default_stream())
+    solve(large, torch.cuda.default_stream())  # (its counters' memory is free again)
+    for _ in range(3):
+        r, x = solve(small, side)
+        assert r.iterations == idle_r.iterations == 6
+        assert np.array_equal(x, idle)
