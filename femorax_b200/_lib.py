@@ -159,6 +159,7 @@ PROTOTYPES = {
     "fx_solver_destroy": (None, [vp]),
     "fx_solver_setup": (C.c_int, [vp, fx_coeffs, vp]),
     "fx_solver_set_inner_tolerance": (C.c_int, [vp, C.c_double]),
+    "fx_solver_set_wait_limit": (C.c_int, [vp, C.c_int32]),
     "fx_solver_solve": (C.c_int, [vp, vp, vp, C.POINTER(fx_solve_result), vp]),
     "fx_solver_newmark": (C.c_int, [vp, vp, vp, vp, vp, C.c_double, C.c_double, C.c_double, C.c_int32, C.c_double,
                                     C.c_int32, C.POINTER(C.c_int32), C.POINTER(fx_solve_result), vp]),
@@ -174,6 +175,7 @@ PROTOTYPES = {
     "fx_explicit_record": (C.c_int, [vp, C.c_int32, vp, C.c_int32]),
     "fx_force_get_launches": (C.c_int, [vp, C.POINTER(C.c_int32)]),
     "fx_nbatch_set_inner": (C.c_int, [vp, C.c_int32, C.c_double]),
+    "fx_nbatch_set_wait_limit": (C.c_int, [vp, C.c_int32]),
     "fx_motions_create": (C.c_int, [C.POINTER(vp)]),
     "fx_motions_destroy": (C.c_int, [vp]),
     "fx_motions_add": (C.c_int, [vp, C.c_int32, C.c_double, p_f64, p_f64, C.c_int32, C.c_double, C.c_double,
@@ -197,6 +199,7 @@ PROTOTYPES = {
     "fx_engine_destroy": (None, [vp]),
     "fx_engine_set_precision": (C.c_int, [vp, C.c_int32]),
     "fx_engine_set_persistent": (C.c_int, [vp, C.c_int32]),
+    "fx_engine_set_wait_limit": (C.c_int, [vp, C.c_int32]),
     "fx_math_eval": (C.c_int, [C.c_int32, vp, vp, vp, C.c_int64, vp]),
     "fx_server_create": (C.c_int, [vp, C.c_int32, C.c_int64, C.c_int32, C.c_int32, C.POINTER(vp)]),
     "fx_server_destroy": (None, [vp]),

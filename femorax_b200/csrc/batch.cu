@@ -498,7 +498,7 @@ template <class TI>
 __global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<TI>)
     k_b_fused(double* sc, int* fl, TI* p, const TI* ap, const TI* inv, TI* d, TI* rr,
               const int* __restrict__ chunk_slot, const SlotDev* __restrict__ sd, int lanes, double* part, int64_t ld,
-              unsigned long long* bar) {
+              unsigned long long* bar, int polls) {
   const int64_t c = blockIdx.x, begin = c * kChunk;
   const int s = slot_of_chunk(chunk_slot, c);
   if (s < 0 || fl[s * NFL + F_DONE]) return;  // (the same for the slot's blocks)
@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<TI>)
   const int64_t left = S.off + S.n - begin;
   const int it = f[F_ITERS];
   cgf::Chunk<TI> a{p, ap, inv, d, rr, begin, static_cast<int>(left < kChunk ? left : kChunk), lanes, c - S.c0, S.nc,
-                   part + S.c0, ld, bar + 2 * s, cs[S_RZ], cs[S_TOL], it, f[F_MAXIT]};
+                   part + S.c0, ld, bar + 2 * s, cs[S_RZ], cs[S_TOL], it, f[F_MAXIT], polls};
   const cgf::Sums o = cgf::iterate(a);
   if (o.state == cgf::kGaveUp && threadIdx.x == 0) f[F_GAVE_UP] = f[F_DONE] = 1;
   if (a.c != 0 || threadIdx.x != 0 || o.state == cgf::kGaveUp) return;
@@ -606,6 +606,7 @@ struct Engine {
   DeviceArray<int> chunk_slot;
   DeviceArray<double> part;  // [3][nchunks]
   DeviceArray<unsigned long long> meet;  // per slot: the fused iteration's two meetings (0 at admission)
+  int polls = cgf::kPolls;               // of a meeting before a block gives up
   DeviceArray<double> sc;
   DeviceArray<int> fl, used_dev, zeros;
   DeviceArray<unsigned> cnt;  // per slot: chunks counted by the fused reductions (0 between launches)
@@ -714,7 +715,7 @@ struct Engine {
     static const int64_t fused_chunks = cgf::capacity(k_b_fused<TI>);  // (thread-safe)
     if (high <= (beside_lanes ? fused_chunks / 4 : fused_chunks)) {  // one launch, every chunk resident
       cgf::launch(k_b_fused<TI>, high, cs, sc.ptr, fl.ptr, p, ap, iv, d, rr, chunk_slot.ptr, sd_dev.ptr, o.lanes,
-                  part.ptr, nchunks, meet.ptr);
+                  part.ptr, nchunks, meet.ptr, polls);
     } else if (high <= kBlockChunks) {  // a block per chunk
       const unsigned gb = static_cast<unsigned>(high);
       k_b_pap<TI, true><<<gb, kChunkBlock, 0, cs>>>(p, ap, high, nchunks, chunk_slot.ptr, sd_dev.ptr, fl.ptr, o.lanes,
@@ -1030,6 +1031,18 @@ int fx_engine_set_persistent(fx_engine* e, int32_t on) {
       e->e.graph = nullptr;
     }
     e->e.persistent = on != 0;
+  });
+}
+
+int fx_engine_set_wait_limit(fx_engine* e, int32_t polls) {
+  return guard([&] {
+    if (!e || polls < 0) throw fx::Error(FX_E_INVALID, "fx_engine_set_wait_limit: bad arguments");
+    FX_CUDA(cudaSetDevice(e->e.device));
+    if (e->e.graph) {  // the inner iterations' graph holds the limit
+      cudaGraphExecDestroy(e->e.graph);
+      e->e.graph = nullptr;
+    }
+    e->e.polls = polls;
   });
 }
 

@@ -25,8 +25,9 @@
 namespace fx {
 namespace cgf {
 
-// Polls of a meeting before a block gives up (a second or more): every block of the launch is
-// resident, so a meeting ends as soon as the slowest block has summed its chunk.
+// Polls of a meeting before a block gives up (a second or more) unless the caller sets another limit:
+// every block of the launch is resident, so a meeting ends as soon as the slowest block has summed its
+// chunk.
 constexpr int kPolls = 1 << 22;
 
 enum : int { kGoOn = 0, kConverged, kLimit, kIndefinite, kGaveUp };
@@ -41,9 +42,9 @@ __device__ __forceinline__ unsigned long long arrive(unsigned long long* cnt, un
   return ticket + (n - rest);
 }
 // Waits until the count is reached; false when it gives up.
-__device__ __forceinline__ bool wait(unsigned long long* cnt, unsigned long long target) {
+__device__ __forceinline__ bool wait(unsigned long long* cnt, unsigned long long target, int polls) {
   unsigned long long now;
-  for (int i = 0; i < kPolls; ++i) {
+  for (int i = 0; i < polls; ++i) {
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(cnt) : "memory");
     if (now >= target) return true;
   }
@@ -110,6 +111,7 @@ struct Chunk {
   unsigned long long* bar;  // the solve's two meetings
   double rz, tol;
   int it, max_it;  // iterations done so far, and their limit
+  int polls;       // of a meeting before a block gives up
 };
 struct Sums {
   double pap, rr, rz;
@@ -213,7 +215,7 @@ __device__ __forceinline__ Sums iterate(const Chunk<T>& a) {
       }
     }
     if (warp <= turn) {
-      if (lane == 0) met[turn + warp] = a.nc == 1 || wait(&a.bar[turn], target);
+      if (lane == 0) met[turn + warp] = a.nc == 1 || wait(&a.bar[turn], target, a.polls);
       __syncwarp();
       const double s = level(col, static_cast<int>(a.nc), a.lanes, lane);
       if (lane == 0) sum[turn + warp] = s;

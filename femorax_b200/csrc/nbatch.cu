@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(256)
 template <class T>
 __global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<T>)
     k_nb_fused(double* sc, int* fl, T* p, const T* ap, const T* inv, T* du, T* rr, const int* __restrict__ owner,
-               const Range* __restrict__ rg, int lanes, double* part, unsigned long long* bar) {
+               const Range* __restrict__ rg, int lanes, double* part, unsigned long long* bar, int polls) {
   const int64_t c = blockIdx.x, begin = c * kChunk;
   const int s = owner[c];
   if (s < 0 || fl[s * NNF + G_CG_DONE]) return;  // (the same for the instance's blocks)
@@ -465,7 +465,8 @@ __global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<T>)
   const Range r = rg[s];
   const int it = f[G_CG_ITERS];
   cgf::Chunk<T> a{p, ap, inv, du, rr, begin, static_cast<int>(chunk_len(r, begin)), lanes, c - r.c0, r.nc,
-                  part + r.c0, gridDim.x, bar + 2 * s, cs[N_RZ], cs[N_TOL], it, f[G_CG_MAXIT]};
+                  part + r.c0, gridDim.x, bar + 2 * s, cs[N_RZ], cs[N_TOL], it, f[G_CG_MAXIT],
+                  polls};
   const cgf::Sums o = cgf::iterate(a);
   if (o.state == cgf::kGaveUp && threadIdx.x == 0) f[G_GAVE_UP] = f[G_CG_DONE] = 1;
   if (a.c != 0 || threadIdx.x != 0 || o.state == cgf::kGaveUp) return;
@@ -672,6 +673,7 @@ struct NBatch {
   DeviceArray<int> fl;
   DeviceArray<unsigned> cnt;  // per instance: chunks counted by the fused reductions (0 between launches)
   DeviceArray<unsigned long long> meet;  // per instance: the fused iteration's two meetings
+  int polls = cgf::kPolls;               // of a meeting before a block gives up
   DeviceArray<int> passes;    // the CG loop graph's pass count
   int* fl_h = nullptr;
   double* sc_h = nullptr;
@@ -684,8 +686,7 @@ struct NBatch {
   cudaGraphExec_t graph32 = nullptr;
 
   ~NBatch() {
-    if (graph) cudaGraphExecDestroy(graph);
-    if (graph32) cudaGraphExecDestroy(graph32);
+    drop_graphs();
     if (fl_h) cudaFreeHost(fl_h);
     if (sc_h) cudaFreeHost(sc_h);
     if (ev_in) cudaEventDestroy(ev_in);
@@ -699,7 +700,7 @@ struct NBatch {
     FX_CUDA(cudaMemcpyAsync(sc_h, sc.ptr, sizeof(double) * NNS * count, cudaMemcpyDeviceToHost, cs));
     FX_CUDA(cudaStreamSynchronize(cs));
     if (any(G_GAVE_UP, 1)) {
-      FX_CUDA(cudaMemset(meet.ptr, 0, meet.bytes()));
+      FX_CUDA(cudaMemsetAsync(meet.ptr, 0, meet.bytes(), cs));  // (before the next step's arrivals)
       throw Error(FX_E_TIMEOUT, "batched CG: a block did not reach its instance's reduction");
     }
   }
@@ -717,7 +718,7 @@ struct NBatch {
     static const int64_t fused_chunks = cgf::capacity(k_nb_fused<T>);  // (thread-safe)
     if (nchunks <= fused_chunks) {  // one launch, every chunk resident
       cgf::launch(k_nb_fused<T>, nchunks, cs, sc.ptr, fl.ptr, pv, apv, iv, dv, rv, owner.ptr, rg.ptr, o.lanes,
-                  part.ptr, meet.ptr);
+                  part.ptr, meet.ptr, polls);
     } else if (nchunks <= kBlockChunks) {  // a block per chunk
       const unsigned gb = static_cast<unsigned>(nchunks);
       k_nb_pap<T, true><<<gb, kChunkBlock, 0, cs>>>(pv, apv, nchunks, owner.ptr, rg.ptr, fl.ptr, o.lanes, part.ptr,
@@ -838,6 +839,13 @@ struct NBatch {
       k_nb_ir_correct<<<g, 32 * kWarps, 0, cs>>>(d32.ptr, du.ptr, nchunks, owner.ptr, rg.ptr, fl.ptr);
       k_nb_ir_round_end<<<inst_grid(), 128, 0, cs>>>(fl.ptr, count);
       FX_LAUNCH_CHECK("nbatch_ir_round");
+    }
+  }
+
+  void drop_graphs() {
+    for (cudaGraphExec_t* g : {&graph, &graph32}) {
+      if (*g) cudaGraphExecDestroy(*g);
+      *g = nullptr;
     }
   }
 
@@ -1057,6 +1065,15 @@ int fx_nbatch_set_inner(fx_nbatch* h, int32_t method, double inner_rtol) {
       }
       FX_CUDA(cudaStreamSynchronize(b.cs));
     }
+  });
+}
+
+int fx_nbatch_set_wait_limit(fx_nbatch* h, int32_t polls) {
+  return guard([&] {
+    if (!h || polls < 0) throw fx::Error(FX_E_INVALID, "fx_nbatch_set_wait_limit: bad arguments");
+    FX_CUDA(cudaSetDevice(h->b.device));
+    h->b.drop_graphs();  // (they hold the limit)
+    h->b.polls = polls;
   });
 }
 

@@ -390,7 +390,7 @@ struct PassEnd {
 template <class T>
 __global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<T>)
     k_cg_fused(double* sc, int* fl, T* p, const T* ap, const T* inv, T* x, T* r, int64_t n, int lanes, double* part,
-               unsigned long long* bar, PassEnd end) {
+               unsigned long long* bar, int polls, PassEnd end) {
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
   if (fl[F_DONE]) {  // (the same for every block: it changes after their last meeting only)
     if (lead && end.cap) cudaGraphSetConditional(end.h, 0u);
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<T>)
   const int64_t c = blockIdx.x, nc = gridDim.x, begin = c * kChunk;
   const int it = fl[F_ITERS];
   cgf::Chunk<T> a{p, ap, inv, x, r, begin, static_cast<int>(n - begin < kChunk ? n - begin : kChunk), lanes, c, nc,
-                  part, nc, bar, sc[S_RZ], sc[S_TOL], it, fl[F_MAXIT]};
+                  part, nc, bar, sc[S_RZ], sc[S_TOL], it, fl[F_MAXIT], polls};
   const cgf::Sums o = cgf::iterate(a);
   if (o.state == cgf::kGaveUp && threadIdx.x == 0) {
     fl[F_GAVE_UP] = 1;
@@ -528,6 +528,7 @@ struct Solver {
   DeviceArray<unsigned> counter;  // the fused kernels' last-block counter (0 between launches)
   DeviceArray<double> fpart;              // the fused iteration's chunk sums, three columns
   DeviceArray<unsigned long long> meet;   // and its two meetings' counters
+  int polls = cgf::kPolls;                // of a meeting before a block gives up
   DeviceArray<double> V, Z, wv, hbuf;  // GMRES
   DeviceArray<double> nres, ndu;       // Newton: residual and increment
   DeviceArray<double> nut, nvt, nat;   // Newmark: the last step's u, v, a
@@ -598,7 +599,8 @@ struct Solver {
     auto iteration = [&](const PassEnd& end) {
       apply(pp, aa, fl.ptr + F_DONE);
       if (fused) {
-        cgf::launch(k_cg_fused<T>, nc, cs, sc.ptr, fl.ptr, pp, aa, iv, x, rr, n, lanes, fpart.ptr, meet.ptr, end);
+        cgf::launch(k_cg_fused<T>, nc, cs, sc.ptr, fl.ptr, pp, aa, iv, x, rr, n, lanes, fpart.ptr, meet.ptr,
+                    polls, end);
         return;
       }
       // p.Ap and alpha, then the update, r.r, r.z and beta (each with its levels in the kernel's
@@ -669,7 +671,7 @@ struct Solver {
     FX_CUDA(cudaGraphLaunch(G.exec, cs));
     read_state();
     if (host_flags[F_GAVE_UP]) {
-      FX_CUDA(cudaMemset(meet.ptr, 0, meet.bytes()));
+      FX_CUDA(cudaMemsetAsync(meet.ptr, 0, meet.bytes(), cs));  // (before the next solve's arrivals)
       throw Error(FX_E_TIMEOUT, "CG: a block did not reach the iteration's reduction");
     }
     res->converged = host_flags[F_CONV];
@@ -1236,6 +1238,15 @@ int fx_solver_set_inner_tolerance(fx_solver* s, double inner_rtol) {
   return guard([&] {
     if (!s || !(inner_rtol > 0.0 && inner_rtol < 1.0)) throw fx::Error(FX_E_INVALID, "inner tolerance must be in (0, 1)");
     s->s.inner_rtol = inner_rtol;
+  });
+}
+
+int fx_solver_set_wait_limit(fx_solver* s, int32_t polls) {
+  return guard([&] {
+    if (!s || polls < 0) throw fx::Error(FX_E_INVALID, "fx_solver_set_wait_limit: bad arguments");
+    FX_CUDA(cudaSetDevice(s->s.f->s.device));
+    s->s.drop_graphs();  // (they hold the limit)
+    s->s.polls = polls;
   });
 }
 

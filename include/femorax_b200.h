@@ -29,7 +29,8 @@ extern "C" {
 #define FX_E_NOMEM 3       /* device or host allocation failed */
 #define FX_E_NOT_SPD 4     /* CG met p.Ap <= 0 (SolveResult::indefinite) */
 #define FX_E_DIVERGED 5    /* non-finite values or no convergence */
-#define FX_E_TIMEOUT 6     /* a bounded device wait gave up (the fused CG iteration's reductions) */
+#define FX_E_TIMEOUT 6     /* a bounded device wait gave up (the fused CG iteration's reductions, see the
+                            * set_wait_limit calls): the solve has no result, its handle stays usable */
 #define FX_E_CUDA 7        /* a CUDA runtime error (message in fx_last_error) */
 #define FX_E_UNSTABLE 8    /* an explicit step above the stable step (the stage's io::ModelError) */
 
@@ -346,6 +347,11 @@ void fx_solver_destroy(fx_solver* s);
 int fx_solver_setup(fx_solver* s, fx_coeffs k, void* stream);
 /* FX_SOLVER_IR: the relative tolerance of each inner FP32 solve (default 1e-4). */
 int fx_solver_set_inner_tolerance(fx_solver* s, double inner_rtol);
+/* The polls after which a block of the fused CG iteration stops waiting for the others of its solve
+ * (default 2^22, a second or more; every block is resident, so a wait ends as soon as the slowest has
+ * summed its part). The call then returns FX_E_TIMEOUT and the next one starts afresh. 0 gives up at
+ * every wait. */
+int fx_solver_set_wait_limit(fx_solver* s, int32_t polls);
 int fx_solver_solve(fx_solver* s, const double* b, double* x, fx_solve_result* r, void* stream);
 /* Newton iterations of one quasi-static load step (ImplicitStage's Newton loop without inertia,
  * src/exec/implicit_stage.cpp:118-437): r = f_ext - f_int(u) with every point's material update
@@ -478,6 +484,9 @@ int fx_nbatch_create(const fx_mesh* meshes, int32_t count, int32_t device, fx_so
  * options' tolerance, as fx_solver_newton with an FX_SOLVER_IR solver: FP32 operator on the
  * stored point tangents, FP64 return map and residuals; per instance the same bits). */
 int fx_nbatch_set_inner(fx_nbatch* b, int32_t method, double inner_rtol);
+/* As fx_solver_set_wait_limit; a step that runs out returns FX_E_TIMEOUT with u at the last Newton
+ * iterate and nothing committed. */
+int fx_nbatch_set_wait_limit(fx_nbatch* b, int32_t polls);
 void fx_nbatch_destroy(fx_nbatch* b);
 int fx_nbatch_layout(const fx_nbatch* b, int64_t* offsets, int64_t* equations);
 fx_force* fx_nbatch_force(fx_nbatch* b);
@@ -538,6 +547,8 @@ int fx_engine_set_precision(fx_engine* e, int32_t inner);
 /* The batched apply as one CTA per (slot, tile) work item (on = 0, the default) or as a persistent
  * wave of CTAs taking the items from a counter (on = 1); the same bits either way. */
 int fx_engine_set_persistent(fx_engine* e, int32_t on);
+/* As fx_solver_set_wait_limit. */
+int fx_engine_set_wait_limit(fx_engine* e, int32_t polls);
 int fx_engine_admit(fx_engine* e, fx_force* f, const double* b_host, int32_t* slot);
 int fx_engine_round(fx_engine* e, int32_t* running);
 int fx_engine_finished(fx_engine* e, int32_t slot, int32_t* finished);
