@@ -637,6 +637,7 @@ class SolveResult:
     final_residual: float
     indefinite: bool
     refinements: int = 0
+    status: int = L.FX_OK  # FX_OK, or why it did not converge (FX_E_NOT_SPD, FX_E_DIVERGED, FX_E_TIMEOUT)
 
 
 class LinearSolver:
@@ -664,7 +665,7 @@ class LinearSolver:
         r = L.fx_solve_result()
         check(lib().fx_solver_solve(self._h, _ptr(b), _ptr(x), C.byref(r), _stream(stream)))
         return SolveResult(bool(r.converged), r.iterations, r.rhs_norm, r.initial_residual, r.final_residual,
-                           bool(r.indefinite), r.refinements)
+                           bool(r.indefinite), r.refinements, r.status)
 
     def newton(self, fext, u, tol: float = 1e-6, test: str = "NormUnbalance", max_newton: int = 25, stream=None):
         """Newton iterations of one quasi-static load step (fx_solver_newton) with the stage's
@@ -677,7 +678,7 @@ class LinearSolver:
         check(lib().fx_solver_newton(self._h, _ptr(fext), _ptr(u), t, tol, max_newton, C.byref(it), C.byref(r),
                                      _stream(stream)))
         return it.value, SolveResult(bool(r.converged), r.iterations, r.rhs_norm, r.initial_residual,
-                                     r.final_residual, bool(r.indefinite), r.refinements)
+                                     r.final_residual, bool(r.indefinite), r.refinements, r.status)
 
     def newmark_step(self, fext, u, v, a, dt: float, beta: float = 0.25, gamma: float = 0.5, tol: float = 1e-6,
                      test: str = "NormUnbalance", max_newton: int = 25, stream=None):
@@ -689,7 +690,7 @@ class LinearSolver:
         check(lib().fx_solver_newmark(self._h, _ptr(fext), _ptr(u), _ptr(v), _ptr(a), dt, beta, gamma, t, tol,
                                       max_newton, C.byref(it), C.byref(r), _stream(stream)))
         return it.value, SolveResult(bool(r.converged), r.iterations, r.rhs_norm, r.initial_residual,
-                                     r.final_residual, bool(r.indefinite), r.refinements)
+                                     r.final_residual, bool(r.indefinite), r.refinements, r.status)
 
     def newmark_step_recover(self, fext0, fext1, u, v, a, dt: float, beta: float = 0.25, gamma: float = 0.5,
                              tol: float = 1e-6, test: str = "NormUnbalance", max_newton: int = 25,
@@ -706,7 +707,7 @@ class LinearSolver:
                                               C.byref(r), _stream(stream)))
         return (dict(zip(("attempts", "failed", "retries", "substepped", "newton"), list(st))),
                 SolveResult(bool(r.converged), r.iterations, r.rhs_norm, r.initial_residual, r.final_residual,
-                            bool(r.indefinite), r.refinements))
+                            bool(r.indefinite), r.refinements, r.status))
 
     def newton_recover(self, fext, u, tol: float = 1e-6, test: str = "NormUnbalance", max_newton: int = 25,
                        max_retries: int = 0, stream=None):
@@ -719,7 +720,7 @@ class LinearSolver:
                                              C.byref(r), _stream(stream)))
         return (dict(zip(("attempts", "failed", "retries", "substepped", "newton"), list(st))),
                 SolveResult(bool(r.converged), r.iterations, r.rhs_norm, r.initial_residual, r.final_residual,
-                            bool(r.indefinite), r.refinements))
+                            bool(r.indefinite), r.refinements, r.status))
 
     def __del__(self):
         h = getattr(self, "_h", None)
@@ -855,7 +856,7 @@ class BatchEngine:
         check(lib().fx_engine_retire(self._h, slot, x.ctypes.data_as(L.p_f64), C.byref(r)))
         del self._forces[slot]
         return x, SolveResult(bool(r.converged), r.iterations, r.rhs_norm, r.initial_residual, r.final_residual,
-                              bool(r.indefinite), r.refinements)
+                              bool(r.indefinite), r.refinements, r.status)
 
     def slots(self):
         return list(self._forces)
@@ -927,7 +928,7 @@ class BatchedNewton:
         res = (L.fx_solve_result * self.count)()
         check(lib().fx_nbatch_step(self._h, _ptr(fext), _ptr(u), tol, max_newton, it, res, _stream(stream)))
         out = [SolveResult(bool(r.converged), r.iterations, r.rhs_norm, r.initial_residual, r.final_residual,
-                           bool(r.indefinite), r.refinements) for r in res]
+                           bool(r.indefinite), r.refinements, r.status) for r in res]
         return np.array(it[:]), out
 
     def commit_state(self, stream=None):

@@ -54,7 +54,7 @@ enum : int {
   G_OUTER, G_INNER, G_INNER_RAN,
   G_NEED_OUTER,  // due for an outer step (admitted, or corrected and not finished)
   F_BEGIN,       // its inner solve starts in this tick (set by the outer step)
-  F_GAVE_UP,     // a block did not reach a reduction of the fused iteration
+  F_GAVE_UP,     // a block gave up waiting at a reduction of the fused iteration
   NFL = 14
 };
 
@@ -510,7 +510,10 @@ __global__ void __launch_bounds__(kChunkBlock, cgf::kMinBlocks<TI>)
   cgf::Chunk<TI> a{p, ap, inv, d, rr, begin, static_cast<int>(left < kChunk ? left : kChunk), lanes, c - S.c0, S.nc,
                    part + S.c0, ld, bar + 2 * s, cs[S_RZ], cs[S_TOL], it, f[F_MAXIT], polls};
   const cgf::Sums o = cgf::iterate(a);
-  if (o.state == cgf::kGaveUp && threadIdx.x == 0) f[F_GAVE_UP] = f[F_DONE] = 1;
+  if (o.state == cgf::kGaveUp && threadIdx.x == 0) {  // the slot has ended: no correction, no further round
+    f[F_GAVE_UP] = f[F_DONE] = f[G_FIN] = 1;
+    f[G_INNER_RAN] = 0;
+  }
   if (a.c != 0 || threadIdx.x != 0 || o.state == cgf::kGaveUp) return;
   cs[S_PAP] = o.pap;
   if (o.state == cgf::kIndefinite) {
@@ -819,9 +822,6 @@ struct Engine {
     }
     FX_CUDA(cudaGraphLaunch(graph, cs));
     read_flags();
-    for (int s = 0; s < max_slots; ++s)
-      if (slots[s].used && fl_h[s * NFL + F_GAVE_UP])
-        throw Error(FX_E_TIMEOUT, "batched CG: a block did not reach its slot's reduction");
     // slots that finished leave the work list
     for (int s = 0; s < max_slots; ++s)
       if (slots[s].used && fl_h[s * NFL + G_FIN]) dirty = true;
@@ -917,7 +917,7 @@ struct Engine {
       res->rhs_norm = c[O_BNORM];
       res->initial_residual = c[O_INIT];
       res->final_residual = c[O_RNORM];
-      res->status = f[G_CONV] ? FX_OK : FX_E_DIVERGED;
+      res->status = f[G_CONV] ? FX_OK : f[F_GAVE_UP] ? FX_E_TIMEOUT : FX_E_DIVERGED;
     }
     for (int64_t cc = sl.c0; cc < sl.c0 + sl.nc; ++cc) chunk_slot_h[cc] = -1;
     slots[slot] = Slot{};

@@ -507,7 +507,7 @@ class NativeServer:
                     result = J2Result(mon[:steps].copy(), nit[:steps].astype(np.int64), bool(res.converged))
                 else:
                     result = SolveResult(bool(res.converged), res.iterations, res.rhs_norm, res.initial_residual,
-                                         res.final_residual, bool(res.indefinite), res.refinements)
+                                         res.final_residual, bool(res.indefinite), res.refinements, res.status)
                 served.append(Served(r.id, x, result, t[0], t[1], t[2]))
             return served, wall.value
         finally:

@@ -547,7 +547,8 @@ int fx_engine_set_precision(fx_engine* e, int32_t inner);
 /* The batched apply as one CTA per (slot, tile) work item (on = 0, the default) or as a persistent
  * wave of CTAs taking the items from a counter (on = 1); the same bits either way. */
 int fx_engine_set_persistent(fx_engine* e, int32_t on);
-/* As fx_solver_set_wait_limit. */
+/* As fx_solver_set_wait_limit; a slot whose wait runs out finishes alone (fx_engine_retire gives
+ * FX_E_TIMEOUT in its result's status and its last corrected x), the others go on. */
 int fx_engine_set_wait_limit(fx_engine* e, int32_t polls);
 int fx_engine_admit(fx_engine* e, fx_force* f, const double* b_host, int32_t* slot);
 int fx_engine_round(fx_engine* e, int32_t* running);

@@ -67,3 +67,49 @@ def test_batched_newton(mixed):
         b.step(f, u)
         out.append(u.cpu().numpy())
     assert out[0].any() and np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("inner", ["fp32", "fp64"])
+def test_engine_finishes_the_failed_slots_alone(inner):
+    """The slots of more than one chunk run out and finish with that status; the one-chunk slot, which
+    meets nobody, goes on to its solution; the freed slots then serve the same requests."""
+    prepared = [serving.prepare(serving.Request(i, *size)) for i, size in
+                enumerate(((14, 12, 7), (3, 4, 5), (10, 10, 12)))]
+
+    def engine():
+        return fx.BatchEngine(1 << 20, 8, options=fx.SolveOptions(relative_tolerance=1e-8), inner=inner)
+
+    def run(e, slots):
+        out = {}
+        for _ in range(400):
+            e.round()
+            for s in [s for s in slots if e.finished(s)]:
+                out[slots.pop(s)] = e.retire(s)
+            if not slots:
+                return out
+        raise AssertionError("the engine did not finish")
+
+    e = engine()
+    want = run(e, {e.admit(f, b): i for i, (f, b, _) in enumerate(prepared)})
+    e = engine()
+    L.check(L.lib().fx_engine_set_wait_limit(e._h, 0))
+    got = run(e, {e.admit(f, b): i for i, (f, b, _) in enumerate(prepared)})
+    assert [got[i][1].status for i in range(3)] == [L.FX_E_TIMEOUT, L.FX_OK, L.FX_E_TIMEOUT]
+    assert not got[0][1].converged and got[1][1].converged
+    assert np.array_equal(got[1][0], want[1][0])
+    L.check(L.lib().fx_engine_set_wait_limit(e._h, DEFAULT))
+    again = run(e, {e.admit(f, b): i for i, (f, b, _) in enumerate(prepared)})
+    for i in range(3):
+        assert again[i][1].converged and np.array_equal(again[i][0], want[i][0]), i
+
+
+def test_server_reports_the_failed_request():
+    """Both loops serve the other requests and give the failed one's status."""
+    stream = [serving.Request(0, 14, 12, 7), serving.Request(1, 3, 4, 5)]
+    for loop in (serving.Server, serving.NativeServer):
+        e = fx.BatchEngine(1 << 20, 8, options=fx.SolveOptions(relative_tolerance=1e-8))
+        L.check(L.lib().fx_engine_set_wait_limit(e._h, 0))
+        served, _ = loop(e, hbm_budget=1 << 34).run(stream, realtime=False)
+        by_id = {s.id: s.result for s in served}
+        assert by_id[0].status == L.FX_E_TIMEOUT and not by_id[0].converged, loop
+        assert by_id[1].converged, loop
