@@ -422,6 +422,7 @@ int fx_force_set_general_mode(fx_force* f, int32_t mode) {
   return guarded([&] {
     FX_REQUIRE(f && (mode == FX_GENERAL_EXACT || mode == FX_GENERAL_FAST), "fx_force_set_general_mode: bad arguments");
     f->s.fast_general = mode == FX_GENERAL_FAST;
+    ++f->s.forms;
   });
 }
 
@@ -432,6 +433,7 @@ int fx_force_set_path(fx_force* f, int32_t path) {
     if (path == FX_PATH_BOX && !f->s.box.qualifies)
       throw fx::Error(FX_E_UNSUPPORTED, "the box path needs a structured grid of equal boxes: " + f->s.box.why_not);
     f->s.path = path;
+    ++f->s.forms;
   });
 }
 
@@ -456,6 +458,7 @@ int fx_force_set_launch(fx_force* f, int32_t variant, int32_t kz) {
     FX_REQUIRE(f, "fx_force_set_launch: null handle");
     if (!f->s.box.qualifies) throw fx::Error(FX_E_UNSUPPORTED, "no box plan: " + f->s.box.why_not);
     fx::box_set_launch(f->s, variant, kz);
+    ++f->s.forms;
   });
 }
 
@@ -484,6 +487,7 @@ int fx_force_tune(fx_force* f, void* stream) {
   return guarded([&] {
     FX_REQUIRE(f, "fx_force_tune: null handle");
     if (f->s.box.qualifies) fx::box_autotune(f->s, static_cast<cudaStream_t>(stream));
+    ++f->s.forms;
   });
 }
 

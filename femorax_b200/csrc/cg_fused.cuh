@@ -155,8 +155,7 @@ __device__ __forceinline__ void store_pairs(T* v, int len, const T (&in)[kChunkP
 }
 
 // The iteration of this block's chunk (all 256 threads); the sums and the state are the same in every
-// thread of every block of the solve. The solver's vectors are aligned to pairs; x may be the caller's
-// and is read entry by entry. The two reductions are two turns of one loop: straight-line code that
+// thread of every block of the solve. The solver's vectors are aligned to pairs. The two reductions are two turns of one loop: straight-line code that
 // runs once per launch costs more in instruction fetches than in issue.
 template <class T>
 __device__ __forceinline__ Sums iterate(const Chunk<T>& a) {

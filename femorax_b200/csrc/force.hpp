@@ -189,6 +189,7 @@ struct ForceState {
   bool any_alpha = false;  // a parameter set with mass-proportional damping
   bool all_soil = false;   // every parameter set bound to a multi-yield soil
   int path = FX_PATH_AUTO;  // requested
+  uint64_t forms = 0;       // counts the calls that change which kernels or buffers the operator runs on
   BoxPlan box;
   // work vectors (host-buffer apply, solvers)
   DeviceArray<double> wx, wy;

@@ -171,6 +171,7 @@ int fx_force_set_pimy(fx_force* f, int32_t set, const fx_pimy* m) {
       s.soil_sd.alloc(static_cast<size_t>(6) * 8 * s.P);
     if (q.rho != m->p.rho)
       throw fx::Error(FX_E_INVALID, "fx_force_set_pimy: the set's density (its masses) differs from the material's");
+    ++s.forms;
     const int need = fx::pimy::nstate(m->p.ns);
     const int64_t P = s.P;
     if (need > s.pimy_nstate) {  // (re)allocate the point arrays; earlier bindings start again

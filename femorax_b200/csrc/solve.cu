@@ -437,6 +437,15 @@ __global__ void k_cg_cond(cudaGraphConditionalHandle h, const int* __restrict__ 
   cudaGraphSetConditional(h, (!fl[F_DONE] && c < cap) ? 1u : 0u);
 }
 
+// out = x, unless a wait gave up
+template <class T>
+__global__ void k_give(const T* __restrict__ x, T* __restrict__ out, int64_t n, const int* __restrict__ fl) {
+  if (fl[F_GAVE_UP]) return;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    out[i] = x[i];
+}
+
 __global__ void k_count_zero(const double* __restrict__ d, int64_t n, int* count) {
   int local = 0;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
@@ -530,25 +539,23 @@ struct Solver {
   DeviceArray<unsigned long long> meet;   // and its two meetings' counters
   int polls = cgf::kPolls;                // of a meeting before a block gives up
   DeviceArray<double> V, Z, wv, hbuf;  // GMRES
-  DeviceArray<double> nres, ndu;       // Newton: residual and increment
+  DeviceArray<double> nres, ndu;       // Newton: residual and increment (any FP64 CG's x)
   DeviceArray<double> nut, nvt, nat;   // Newmark: the last step's u, v, a
   DeviceArray<double> cu, cv, ca, fx_t;  // recovery: the committed u, v, a of an attempt; its load
   DeviceArray<double> ct_j2, ct_pimy, ct_pdmy;  // recovery: the points' tangents before an attempt
   int* host_flags = nullptr;           // pinned
   double* host_sc = nullptr;           // pinned
-  // The CG loop graph of the last solve per precision (0: FP64, 1: FP32 inner), kept for the next
-  // solve on the same vectors (the Newton and Newmark loops, refinement rounds, whose iteration limits
-  // differ: the limit is a device value): capturing and instantiating it costs as much as tens of
-  // iterations. Dropped when setup changes the
-  // coefficients (the layered tables are kernel parameters captured with it).
-  struct CgGraph {
-    cudaGraphExec_t exec = nullptr;
-    const void* key[5] = {};
-  } cg_graph[2];
+  // The CG loop graph per precision (0: FP64, 1: FP32 inner), kept for the next solve (the iteration
+  // limit is a device value): capturing and instantiating it costs as much as tens of iterations. It
+  // holds the solver's own vectors only, so a solve with another x runs the same graph. Dropped when
+  // setup changes the coefficients (the layered tables are kernel parameters captured with it) or a
+  // call on the force changed the operator's form (path, mode, launch shape, materials, tangent).
+  cudaGraphExec_t cg_graph[2] = {nullptr, nullptr};
+  uint64_t graph_forms = 0;  // the operator's form they were captured in
   void drop_graphs() {
     for (auto& g : cg_graph) {
-      if (g.exec) cudaGraphExecDestroy(g.exec);
-      g = CgGraph{};
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
     }
   }
   ~Solver() {
@@ -575,9 +582,17 @@ struct Solver {
     FX_CUDA(cudaStreamSynchronize(cs));
   }
 
-  // Jacobi-PCG on vectors of type T (double: the plain solve; float: the inner solve of IR).
+  // Jacobi-PCG on vectors of type T (double: the plain solve, ndu; float: the inner solve of IR, d32), on
+  // the solver's own vectors. `out`: where the iterate goes at the end, unless a wait gave up.
   template <class T>
-  void cg(const T* b, T* x, T* rr, T* pp, T* aa, const T* iv, double rtol, double atol, int max_it, fx_solve_result* res) {
+  void cg(const T* b, double rtol, double atol, int max_it, fx_solve_result* res, T* out = nullptr) {
+    T *x, *rr, *pp, *aa;
+    const T* iv;
+    if constexpr (sizeof(T) == 8) {
+      x = ndu.ptr, rr = r.ptr, pp = p.ptr, aa = ap.ptr, iv = inv.ptr;
+    } else {  // (the CG residual needs a buffer of its own: x0's storage)
+      x = d32.ptr, rr = reinterpret_cast<float*>(x0.ptr), pp = p32.ptr, aa = ap32.ptr, iv = inv32.ptr;
+    }
     const int lanes = o.lanes;
     const int64_t nc = chunks_of(n);
     auto apply = [&](const T* xin, T* yout, const int* skip) {
@@ -623,14 +638,12 @@ struct Solver {
     // The iterations run as one graph: a while node whose body is kCgPass iterations and the
     // condition kernel, so the device loops until the solve is done with no host round trip.
     // The begin above ran eagerly (its apply builds lazy state and this solver's coefficient
-    // tables); a new graph is captured when the vectors differ from the last solve's.
-    CgGraph& G = cg_graph[sizeof(T) == 4 ? 1 : 0];
-    const void* key[5] = {x, rr, pp, aa, iv};
-    if (G.exec && std::memcmp(G.key, key, sizeof key) != 0) {
-      cudaGraphExecDestroy(G.exec);
-      G = CgGraph{};
-    }
-    if (!G.exec) {
+    // tables).
+    const uint64_t form = 2 * f->s.forms + (f->s.initial ? 1 : 0);
+    if (graph_forms != form) drop_graphs();
+    graph_forms = form;
+    cudaGraphExec_t& G = cg_graph[sizeof(T) == 4 ? 1 : 0];
+    if (!G) {
       cudaGraph_t g = nullptr;
       FX_CUDA(cudaGraphCreate(&g, 0));
       try {
@@ -657,18 +670,21 @@ struct Solver {
           throw;
         }
         FX_CUDA(cudaStreamEndCapture(cs, &body));
-        FX_CUDA(cudaGraphInstantiate(&G.exec, g, 0));
+        FX_CUDA(cudaGraphInstantiate(&G, g, 0));
       } catch (...) {
-        if (G.exec) cudaGraphExecDestroy(G.exec);
-        G = CgGraph{};
+        if (G) cudaGraphExecDestroy(G);
+        G = nullptr;
         cudaGraphDestroy(g);
         throw;
       }
       cudaGraphDestroy(g);
-      std::memcpy(G.key, key, sizeof key);
     }
     FX_CUDA(cudaMemsetAsync(passes.ptr, 0, sizeof(int), cs));
-    FX_CUDA(cudaGraphLaunch(G.exec, cs));
+    FX_CUDA(cudaGraphLaunch(G, cs));
+    if (out) {
+      k_give<T><<<ew(n), 256, 0, cs>>>(x, out, n, fl.ptr);
+      FX_LAUNCH_CHECK("cg_give");
+    }
     read_state();
     if (host_flags[F_GAVE_UP]) {
       FX_CUDA(cudaMemsetAsync(meet.ptr, 0, meet.bytes(), cs));  // (before the next solve's arrivals)
@@ -680,6 +696,12 @@ struct Solver {
     res->rhs_norm = host_sc[S_RHS];
     res->initial_residual = host_sc[S_INIT];
     res->final_residual = host_sc[S_RNORM];
+  }
+
+  // the plain solve from the caller's x, and back to it
+  void cg_from(const double* b, double* x, fx_solve_result* res) {
+    FX_CUDA(cudaMemcpyAsync(ndu.ptr, x, sizeof(double) * n, cudaMemcpyDeviceToDevice, cs));
+    cg<double>(b, o.rtol, o.atol, o.max_iterations, res, x);
   }
 
   void gmres(const double* b, double* x, fx_solve_result* res);
@@ -836,9 +858,7 @@ void Solver::ir(const double* b, double* x, fx_solve_result* res) {
     k_zero_f32<<<ew(n), 256, 0, cs>>>(d32.ptr, n);
     FX_LAUNCH_CHECK("ir_inner_setup");
     fx_solve_result ri{};
-    // the FP32 rhs lives in r32; the CG residual vector needs its own buffer: reuse x0 as FP32 storage
-    float* rr32 = reinterpret_cast<float*>(x0.ptr);
-    cg<float>(r32.ptr, d32.ptr, rr32, p32.ptr, ap32.ptr, inv32.ptr, inner_rtol, 0.0, o.max_iterations - inner_total, &ri);
+    cg<float>(r32.ptr, inner_rtol, 0.0, o.max_iterations - inner_total, &ri);
     inner_total += ri.iterations;
     k_add_f32<<<ew(n), 256, 0, cs>>>(d32.ptr, x, n);
     FX_LAUNCH_CHECK("ir_correct");
@@ -891,7 +911,7 @@ int Solver::newton(const double* fext, double* u, int test, double tol, int max_
     FX_CUDA(cudaMemsetAsync(ndu.ptr, 0, sizeof(double) * n, cs));
     fx_solve_result lin{};
     if (method == FX_SOLVER_IR) ir(nres.ptr, ndu.ptr, &lin);  // FP32 CG on the tangent, FP64 refinement
-    else cg<double>(nres.ptr, ndu.ptr, r.ptr, p.ptr, ap.ptr, inv.ptr, o.rtol, o.atol, o.max_iterations, &lin);
+    else cg<double>(nres.ptr, o.rtol, o.atol, o.max_iterations, &lin);
     k_add64<<<ew(n), 256, 0, cs>>>(ndu.ptr, u, n);
     FX_LAUNCH_CHECK("newton_update");
     res->iterations += lin.iterations;
@@ -964,7 +984,7 @@ int Solver::newmark(const double* fext, double* u, double* v, double* a, double 
     FX_CUDA(cudaMemsetAsync(ndu.ptr, 0, sizeof(double) * n, cs));
     fx_solve_result lin{};
     if (method == FX_SOLVER_IR) ir(nres.ptr, ndu.ptr, &lin);
-    else cg<double>(nres.ptr, ndu.ptr, r.ptr, p.ptr, ap.ptr, inv.ptr, o.rtol, o.atol, o.max_iterations, &lin);
+    else cg<double>(nres.ptr, o.rtol, o.atol, o.max_iterations, &lin);
     newmark_update(n, ndu.ptr, u, v, a, c2, c3, cs);
     res->iterations += lin.iterations;
     res->refinements += lin.refinements;
@@ -1275,14 +1295,14 @@ int fx_solver_solve(fx_solver* h, const double* b, double* x, fx_solve_result* r
     FX_CUDA(cudaStreamWaitEvent(s.cs, s.ev_in, 0));
     switch (s.method) {
       case FX_SOLVER_CG:
-        s.cg<double>(b, x, s.r.ptr, s.p.ptr, s.ap.ptr, s.inv.ptr, s.o.rtol, s.o.atol, s.o.max_iterations, r);
+        s.cg_from(b, x, r);
         break;
       case FX_SOLVER_GMRES:
         s.gmres(b, x, r);
         break;
       case FX_SOLVER_KRYLOV: {
         FX_CUDA(cudaMemcpyAsync(s.x0.ptr, x, sizeof(double) * s.n, cudaMemcpyDeviceToDevice, s.cs));
-        s.cg<double>(b, x, s.r.ptr, s.p.ptr, s.ap.ptr, s.inv.ptr, s.o.rtol, s.o.atol, s.o.max_iterations, r);
+        s.cg_from(b, x, r);
         if (r->indefinite) {
           const int cg_it = r->iterations;
           FX_CUDA(cudaMemcpyAsync(x, s.x0.ptr, sizeof(double) * s.n, cudaMemcpyDeviceToDevice, s.cs));

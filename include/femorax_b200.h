@@ -349,8 +349,8 @@ int fx_solver_setup(fx_solver* s, fx_coeffs k, void* stream);
 int fx_solver_set_inner_tolerance(fx_solver* s, double inner_rtol);
 /* The polls after which a block of the fused CG iteration stops waiting for the others of its solve
  * (default 2^22, a second or more; every block is resident, so a wait ends as soon as the slowest has
- * summed its part). The call then returns FX_E_TIMEOUT and the next one starts afresh. 0 gives up at
- * every wait. */
+ * summed its part). The call then returns FX_E_TIMEOUT (fx_solver_solve: x as it was given, or an
+ * FX_SOLVER_IR solve's last corrected x) and the next one starts afresh. 0 gives up at every wait. */
 int fx_solver_set_wait_limit(fx_solver* s, int32_t polls);
 int fx_solver_solve(fx_solver* s, const double* b, double* x, fx_solve_result* r, void* stream);
 /* Newton iterations of one quasi-static load step (ImplicitStage's Newton loop without inertia,

@@ -32,10 +32,11 @@ def test_solver(solver):
             L.check(L.lib().fx_solver_set_wait_limit(s._h, polls))
             if polls:
                 continue
-            x = torch.zeros(n, dtype=torch.float64, device=DEV)
+            x = torch.ones(n, dtype=torch.float64, device=DEV)
             with pytest.raises(fx.FxError) as e:
                 s.solve(b, x)
             assert e.value.code == L.FX_E_TIMEOUT
+            assert (x == 1.0).all()
         x = torch.zeros(n, dtype=torch.float64, device=DEV)
         assert s.solve(b, x).converged
         out.append(x.cpu().numpy())
