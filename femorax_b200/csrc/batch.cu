@@ -715,7 +715,8 @@ struct Engine {
   template <class TI>
   void inner_iteration_t(const unsigned char* inst, TI* p, TI* ap, const TI* iv, TI* d, TI* rr) {
     box_batch_apply(sizeof(TI) == 4, inst, work.ptr, nwork, kz, persistent ? queue.ptr : nullptr, cs);
-    static const int64_t fused_chunks = cgf::capacity(k_b_fused<TI>);  // (thread-safe)
+    static PerDevice<int64_t> known;
+    const int64_t fused_chunks = cgf::capacity(known, k_b_fused<TI>);
     if (high <= (beside_lanes ? fused_chunks / 4 : fused_chunks)) {  // one launch, every chunk resident
       cgf::launch(k_b_fused<TI>, high, cs, sc.ptr, fl.ptr, p, ap, iv, d, rr, chunk_slot.ptr, sd_dev.ptr, o.lanes,
                   part.ptr, nchunks, meet.ptr, polls);

@@ -542,19 +542,18 @@ constexpr int kBatchBX = 16, kBatchBY = 8;
 template <class T>
 constexpr int kBatchMinB = sizeof(T) == 4 ? 6 : 4;  // FP32 fits 6 CTAs per SM without spills
 
-// CTAs of the batch kernel that are resident at once (set once, thread-safe: serving threads launch
-// this concurrently)
+// CTAs of the batch kernel that are resident at once on the current device
 template <class T>
 int batch_resident() {
   using S = Smem<kBatchBX, kBatchBY, T, 0, kPerSet>;
   auto kern = k_box_batch<kBatchBX, kBatchBY, T, 0, kBatchMinB<T>>;
-  static const int resident = [&] {
+  static PerDevice<int> resident;
+  return resident.get(current_device(), [&] {
     int r = 0;
     FX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(S::bytes)));
     FX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kern, kBatchBX * kBatchBY, S::bytes));
     return std::max(r, 1) * num_sms();
-  }();
-  return resident;
+  });
 }
 
 template <class T>

@@ -253,12 +253,15 @@ __device__ __forceinline__ Sums iterate(const Chunk<T>& a) {
 template <class T>
 constexpr int kMinBlocks = sizeof(T) == 8 ? 2 : 4;
 
-// Chunks (blocks) that fit on the device at once for kernel `kern`.
+// Chunks (blocks) that fit on the current device at once for kernel `kern` (`known`: a static of the
+// launch site).
 template <class Kernel>
-int64_t capacity(Kernel kern) {
-  int per_sm = 0;
-  FX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kChunkBlock, 0));
-  return static_cast<int64_t>(per_sm) * num_sms();
+int64_t capacity(PerDevice<int64_t>& known, Kernel kern) {
+  return known.get(current_device(), [&] {
+    int per_sm = 0;
+    FX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kChunkBlock, 0));
+    return static_cast<int64_t>(per_sm) * num_sms();
+  });
 }
 
 // A cooperative launch of `blocks` blocks (all resident together, or the launch fails).

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "host.hpp"
+#include "per_device.hpp"
 
 namespace fx {
 
@@ -52,14 +53,30 @@ struct DeviceArray {
   size_t bytes() const { return n * sizeof(T); }
 };
 
+inline int current_device() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return dev;
+}
+
 inline int num_sms() {
-  static int sms = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
+  static PerDevice<int> sms;
+  const int dev = current_device();
+  return sms.get(dev, [dev] {
+    int v = 0;
     cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
     return v > 0 ? v : 148;
-  }();
-  return sms;
+  });
+}
+
+// The kernel's limit of dynamic shared memory on the current device (set once per device; `set`: a
+// static of the launch site).
+template <class Kernel>
+void allow_shared(PerDevice<bool>& set, Kernel kern, size_t bytes) {
+  set.get(current_device(), [&] {
+    FX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+    return true;
+  });
 }
 
 inline unsigned grid_for(int64_t n, int block) { return static_cast<unsigned>((n + block - 1) / block); }

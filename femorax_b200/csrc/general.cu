@@ -212,11 +212,8 @@ __global__ void __launch_bounds__(points::kThreads, 2)
 template <bool MASS>
 void launch_points_apply(ForceState& s, const double k[3], const double* x, cudaStream_t st, const int* skip) {
   constexpr int bytes = static_cast<int>(sizeof(points::Stage<1, MASS ? 2 : 1>));
-  static const bool once = [] {  // (thread-safe)
-    FX_CUDA(cudaFuncSetAttribute(k_points_apply<MASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    return true;
-  }();
-  (void)once;
+  static PerDevice<bool> set;
+  allow_shared(set, k_points_apply<MASS>, bytes);
   k_points_apply<MASS><<<grid_for(s.count, points::kEl), points::kThreads, bytes, st>>>(
       s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr, s.params.ptr, s.N, s.P, s.count, k[0], k[1], k[2], x,
       s.slots.ptr, skip, s.j2_tan.ptr, s.initial);
@@ -586,11 +583,8 @@ __global__ void __launch_bounds__(points::kThreads, 2)
 void soil_force(ForceState& s, const double* v, const double* sig, int kind, cudaStream_t st) {
   if (!s.any_alpha && !s.soil_sd.ptr) {
     constexpr int bytes = static_cast<int>(sizeof(points::Stage<1, 1>));
-    static const bool once = [] {  // (thread-safe)
-      FX_CUDA(cudaFuncSetAttribute(k_soil_force_points, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-      return true;
-    }();
-    (void)once;
+    static PerDevice<bool> set;
+    allow_shared(set, k_soil_force_points, bytes);
     k_soil_force_points<<<grid_for(s.count, points::kEl), points::kThreads, bytes, st>>>(
         s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr, s.params.ptr, s.N, s.P, s.count, v, sig, s.slots.ptr, kind);
   } else {

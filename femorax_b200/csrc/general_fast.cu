@@ -150,20 +150,9 @@ bool general_fast_applies(const ForceState& s) {
   return true;
 }
 
-// the kernels' shared-memory limit, set once (thread-safe)
-void fast_attributes() {
-  static const bool once = [] {
-    FX_CUDA(cudaFuncSetAttribute(k_apply_fast, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 sizeof(points::Stage<1, 1>)));
-    FX_CUDA(cudaFuncSetAttribute(k_force_fast, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 sizeof(points::Stage<2, 1>)));
-    return true;
-  }();
-  (void)once;
-}
-
 void general_apply_fast(ForceState& s, const double k[3], const double* x, double* y, cudaStream_t st, const int* skip) {
-  fast_attributes();
+  static PerDevice<bool> set;
+  allow_shared(set, k_apply_fast, sizeof(points::Stage<1, 1>));
   if (s.count > 0)
     k_apply_fast<<<fast_grid(s.count), kThreads, sizeof(points::Stage<1, 1>), st>>>(
         s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr, s.params.ptr, s.N, s.P, s.count, k[0], k[1], k[2], x,
@@ -173,7 +162,8 @@ void general_apply_fast(ForceState& s, const double k[3], const double* x, doubl
 }
 
 void general_force_fast(ForceState& s, const double* u, const double* v, double* f, cudaStream_t st) {
-  fast_attributes();
+  static PerDevice<bool> set;
+  allow_shared(set, k_force_fast, sizeof(points::Stage<2, 1>));
   if (s.count > 0)
     k_force_fast<<<fast_grid(s.count), kThreads, sizeof(points::Stage<2, 1>), st>>>(
         s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr, s.params.ptr, s.N, s.P, s.count, u, v, s.slots.ptr);

@@ -715,7 +715,8 @@ struct NBatch {
   // the vector kernels of one CG iteration (in vectors of type T), in the form for this many chunks
   template <class T>
   void cg_vectors(T* pv, T* apv, const T* iv, T* dv, T* rv) {
-    static const int64_t fused_chunks = cgf::capacity(k_nb_fused<T>);  // (thread-safe)
+    static PerDevice<int64_t> known;
+    const int64_t fused_chunks = cgf::capacity(known, k_nb_fused<T>);
     if (nchunks <= fused_chunks) {  // one launch, every chunk resident
       cgf::launch(k_nb_fused<T>, nchunks, cs, sc.ptr, fl.ptr, pv, apv, iv, dv, rv, owner.ptr, rg.ptr, o.lanes,
                   part.ptr, meet.ptr, polls);

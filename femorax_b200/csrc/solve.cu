@@ -609,7 +609,8 @@ struct Solver {
     reduce_partials(w, nc, 2, sc.ptr + S_RR, cs);
     k_cg_start<<<1, 1, 0, cs>>>(sc.ptr, fl.ptr, rtol, atol, max_it);
     FX_LAUNCH_CHECK("cg_start");
-    static const int64_t fused_chunks = cgf::capacity(k_cg_fused<T>);  // (thread-safe)
+    static PerDevice<int64_t> known;
+    const int64_t fused_chunks = cgf::capacity(known, k_cg_fused<T>);
     const bool fused = nc <= fused_chunks;
     auto iteration = [&](const PassEnd& end) {
       apply(pp, aa, fl.ptr + F_DONE);
