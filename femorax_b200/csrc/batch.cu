@@ -624,9 +624,6 @@ struct Engine {
   // persistent wave on 120 static solves with FP32 inner solves, equal with FP64 ones, B200) or as a
   // persistent wave of CTAs taking the items from `queue`.
   bool persistent = false;
-  // The serving loop steps J2 cohorts on other streams beside this engine: a cooperative launch starts
-  // when all its blocks fit at once, so beside them it may take a quarter of the GPU only.
-  bool beside_lanes = false;
   // host state
   struct Slot {
     bool used = false;
@@ -717,7 +714,7 @@ struct Engine {
     box_batch_apply(sizeof(TI) == 4, inst, work.ptr, nwork, kz, persistent ? queue.ptr : nullptr, cs);
     static PerDevice<int64_t> known;
     const int64_t fused_chunks = cgf::capacity(known, k_b_fused<TI>);
-    if (high <= (beside_lanes ? fused_chunks / 4 : fused_chunks)) {  // one launch, every chunk resident
+    if (high <= fused_chunks) {  // one launch, every chunk resident
       cgf::launch(k_b_fused<TI>, high, cs, sc.ptr, fl.ptr, p, ap, iv, d, rr, chunk_slot.ptr, sd_dev.ptr, o.lanes,
                   part.ptr, nchunks, meet.ptr, polls);
     } else if (high <= kBlockChunks) {  // a block per chunk
@@ -1014,14 +1011,6 @@ int fx_engine_create(int32_t device, int64_t capacity, int32_t max_slots, fx_coe
 }
 
 void fx_engine_destroy(fx_engine* e) { delete e; }
-
-void fx_engine_beside_lanes(fx_engine* e) {
-  if (e->e.graph) {  // the inner iterations' graph may hold the other form
-    cudaGraphExecDestroy(e->e.graph);
-    e->e.graph = nullptr;
-  }
-  e->e.beside_lanes = true;
-}
 
 int fx_engine_set_persistent(fx_engine* e, int32_t on) {
   return guard([&] {

@@ -325,6 +325,3 @@ void box_batch_apply(bool f32, const void* inst, const int4* work, int nwork, in
 struct fx_force {
   fx::ForceState s;
 };
-
-// batch.cu: the engine's launches leave room for the serving loop's lanes on other streams
-extern "C" void fx_engine_beside_lanes(fx_engine* e);

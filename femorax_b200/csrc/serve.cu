@@ -403,7 +403,6 @@ int fx_server_create(fx_engine* engine, int32_t device, int64_t hbm_budget, int3
   return fx::guard([&] {
     if (!engine || !out || hbm_budget < 0 || max_cohort <= 0 || max_lanes <= 0)
       throw fx::Error(FX_E_INVALID, "fx_server_create: bad arguments");
-    fx_engine_beside_lanes(engine);
     auto* h = new fx_server;
     h->s.engine = engine;
     h->s.device = device;

@@ -3,6 +3,8 @@ argument errors with status codes (no device work: runs without a GPU)."""
 import ctypes as C
 import os
 import re
+import shutil
+import subprocess
 
 import numpy as np
 import pytest
@@ -24,6 +26,15 @@ def test_every_declared_symbol_is_exported():
     missing = [n for n in declared() if not hasattr(lib, n)]
     assert not missing, missing
     assert set(declared()) <= set(L.PROTOTYPES), sorted(set(declared()) - set(L.PROTOTYPES))
+
+
+def test_every_exported_symbol_is_declared():
+    nm = shutil.which("nm")
+    if not nm:
+        pytest.skip("no nm")
+    out = subprocess.run([nm, "-D", "--defined-only", L.LIB_PATH], capture_output=True, text=True, check=True).stdout
+    exported = {line.split()[2] for line in out.splitlines() if len(line.split()) == 3 and line.split()[2].startswith("fx_")}
+    assert exported == set(declared())
 
 
 def test_version_and_errors():
