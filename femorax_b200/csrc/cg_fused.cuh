@@ -182,6 +182,10 @@ __device__ __forceinline__ Sums iterate(const Chunk<T>& a) {
         vr[k] = fma(-alpha, va[k], vr[k]);
         vi[k] = vi[k] * vr[k];
       }
+      if (a.len < kChunk)  // (an infinite alpha makes the zeros past the end NaN)
+#pragma unroll
+        for (int k = 0; k < kChunkPer; ++k)
+          if (pair_at(k / 2) + k % 2 >= a.len) vr[k] = vi[k] = T(0);
       store_pairs(sb, kChunk, vr);
       store_pairs(sa, kChunk, vi);
     }

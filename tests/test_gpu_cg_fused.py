@@ -58,6 +58,30 @@ def test_iterates(size, oracle_mod):
             assert np.array_equal(got[0], got[1])
 
 
+def test_infinite_alpha():
+    """r.z overflows while p.Ap and ||b|| do not: alpha is infinite, and the residual's norm after the
+    step is infinite, as the sums over the vector's own entries give it for any lane count; the chunk's
+    zeros past its end (inf times 0) take no part."""
+    spec = meshes.box_model(7, 9, 8, E=1e-8)
+    force = fx.InternalForce(fx.Model(spec).compile().mesh())
+    n = force.num_equations
+    assert n % 2048
+    op = fx.MatrixFreeOperator(force)
+    d, kz = (torch.zeros(n, dtype=torch.float64, device=DEV) for _ in range(2))
+    op.diagonal(d)
+    z = torch.as_tensor(1.0 + 0.3 * np.random.default_rng(5).random(n), device=DEV)
+    z *= 1.7e154 / float(z @ (d * z)) ** 0.5  # z.Dz = 2.9e308, past the largest double
+    b = d * z
+    op.apply(z, kz)
+    assert torch.isinf(b @ z) and torch.isfinite(z @ kz) and torch.isfinite(b @ b) and bool((kz != 0).all())
+    for lanes in (32, 7):
+        s = fx.ConjugateGradient(fx.SolveOptions(relative_tolerance=1e-10, max_iterations=1, lanes=lanes))
+        s.setup(op)
+        r = s.solve(b, torch.zeros_like(b))
+        assert r.iterations == 1 and not r.converged and not r.indefinite
+        assert r.final_residual == np.inf, (lanes, r.final_residual)
+
+
 def test_created_beside_a_busy_default_stream():
     """A solver's counters start at zero for its own stream's solves also while the default stream, on
     which they are zeroed, still works through other kernels (and the memory held another solver's
