@@ -67,7 +67,8 @@ struct Stage<NX, 0> {
 };
 
 // The block's elements: their edge vectors and their values of x0 (and x1), by all threads; the point
-// tables by eight of them. Elements past `count` stage zeros (their points are not evaluated).
+// tables by eight of them. Elements past `count` stage zeros: a degenerate element, whose points give
+// NaN where a kernel evaluates them (it writes nothing of theirs).
 template <int NX, int NP>
 __device__ __forceinline__ void stage_elements(Stage<NX, NP>& S, const double* __restrict__ coords,
                                                const int32_t* __restrict__ node, const int32_t* __restrict__ eq,
