@@ -540,7 +540,7 @@ struct Solver {
   int polls = cgf::kPolls;                // of a meeting before a block gives up
   DeviceArray<double> V, Z, wv, hbuf;  // GMRES
   DeviceArray<double> nres, ndu;       // Newton: residual and increment (any FP64 CG's x)
-  DeviceArray<double> nut, nvt, nat;   // Newmark: the last step's u, v, a
+  DeviceArray<double> nut, nvt, nat;   // Newmark: the last step's u, v, a (nvt: Newton's zero velocity)
   DeviceArray<double> cu, cv, ca, fx_t;  // recovery: the committed u, v, a of an attempt; its load
   DeviceArray<double> ct_j2, ct_pimy, ct_pdmy;  // recovery: the points' tangents before an attempt
   int* host_flags = nullptr;           // pinned
@@ -881,7 +881,9 @@ void Solver::ir(const double* b, double* x, fx_solve_result* res) {
 // ||f_ext||, the first and last ||r||.
 int Solver::newton(const double* fext, double* u, int test, double tol, int max_newton, fx_solve_result* res) {
   ForceState& fs = f->s;
-  FX_CUDA(cudaMemsetAsync(x0.ptr, 0, sizeof(double) * n, cs));  // velocity 0 (quasi-static)
+  // velocity 0 (quasi-static), in a vector that no linear solve writes (x0 holds the FP32 CG's residual)
+  const double* still = nvt.ptr;
+  FX_CUDA(cudaMemsetAsync(nvt.ptr, 0, sizeof(double) * n, cs));
   auto norm = [&](const double* v) {
     dot_device(w, v, v, n, sc.ptr + S_RR, cs);
     FX_CUDA(cudaMemcpyAsync(host_sc, sc.ptr, sizeof(double) * S_NSCALAR, cudaMemcpyDeviceToHost, cs));
@@ -889,8 +891,8 @@ int Solver::newton(const double* fext, double* u, int test, double tol, int max_
     return std::sqrt(host_sc[S_RR]);
   };
   auto residual = [&]() {  // nres = f_ext - f_int(u)
-    if (fs.use_box_force()) box_force(fs, u, x0.ptr, nres.ptr, cs);
-    else general_force(fs, u, x0.ptr, nres.ptr, cs);
+    if (fs.use_box_force()) box_force(fs, u, still, nres.ptr, cs);
+    else general_force(fs, u, still, nres.ptr, cs);
     k_sub_from<<<ew(n), 256, 0, cs>>>(fext, nres.ptr, n);
     FX_LAUNCH_CHECK("newton_residual");
     return norm(nres.ptr);

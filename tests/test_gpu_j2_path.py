@@ -98,3 +98,30 @@ def test_mixed_precision_newton_on_j2(oracle_mod):
     assert plain.plastic.max() > 0
     assert np.array_equal(mixed.plastic, plain.plastic)
     assert np.max(np.abs(mixed.monitor - plain.monitor)) <= 1e-6 * np.max(np.abs(plain.monitor))
+
+
+@pytest.mark.parametrize("path", ["general", "box"])
+def test_mixed_newton_of_a_damped_mesh_is_quasi_static(path):
+    """Every force evaluation of a load step is at velocity zero, the mixed solver's too: with Rayleigh
+    damping, large loads and loose linear solves (whose FP32 residuals are large numbers), the steps
+    converge and u is the plain Newton's within the residual's tolerance."""
+    spec = fx.meshes.box_model(5, 4, 6, lumped=True)
+    grid = spec.grid
+    if path == "general":
+        spec = fx.meshes.distort(spec, 0.1, seed=3)
+        spec.grid = grid  # (the load's node areas)
+    spec.rayleigh = [fx.meshes.Rayleigh(0.5, 2e-3, 0.0, 0.0, spec.groups[0].etags)]
+    comp = fx.Model(spec).compile()
+    force = fx.InternalForce(comp.mesh())
+    assert force.info()["path"] == path
+    F, _ = top_shear_load(spec, serving.equation_map(comp), 1e9)
+    f = torch.as_tensor(F, device=DEV)
+    got = []
+    for solver in (fx.ConjugateGradient(fx.SolveOptions(relative_tolerance=1e-12)),
+                   fx.MixedPrecisionSolver(fx.SolveOptions(relative_tolerance=1e-3), inner_tolerance=1e-1)):
+        solver.setup(fx.MatrixFreeOperator(force, fx.OperatorCoefficients()))
+        u = torch.zeros_like(f)
+        it, r = solver.newton(f, u, tol=1e-9 * float(f.norm()))
+        assert r.converged and it <= 12, (it, r)
+        got.append(u)
+    assert float((got[1] - got[0]).norm()) <= 1e-6 * float(got[0].norm())
