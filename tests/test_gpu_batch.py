@@ -7,7 +7,7 @@
 - every solution meets the 1e-8 relative FP64 residual, checked here with the FP64 operator, and
   agrees with the plain FP64 CG solution to 1e-6 relative;
 - admission refuses when no slot or no range of chunks is free, and a retire makes room again;
-- the block-per-chunk and warp-per-chunk forms of the CG vector kernels give the same bits.
+- the fused, block-per-chunk and warp-per-chunk forms of the CG vector kernels give the same bits.
 """
 import numpy as np
 import pytest
@@ -85,10 +85,10 @@ def single_ir(force, b, n):
 
 
 def test_block_and_warp_forms_same_bits(prepared):
-    """The CG vector kernels take a block per chunk for vectors of at most 1,024 chunks and a warp
-    per chunk beyond; both sum in the same order. A small mesh batched beside one of more than 1,024
-    chunks runs the engine's warp form, its single solve the block form: the same bits, iterations
-    and rounds; the large mesh matches its own single solve too."""
+    """The CG vector kernels sum in the same order in every form: one fused launch for batches that fit
+    on the GPU, a block per chunk for at most 1,024 chunks, a warp per chunk beyond. A small mesh
+    batched beside one of more than 1,024 chunks runs the engine's warp form, its single solve the
+    fused form: the same bits, iterations and rounds; the large mesh matches its own single solve too."""
     big = serving.Request(9, 100, 100, 70)
     fb, bb, nb = serving.prepare(big)
     assert nb > 1024 * 2048
@@ -103,6 +103,43 @@ def test_block_and_warp_forms_same_bits(prepared):
         assert r.converged and re.converged, rid
         assert np.array_equal(xe, x), rid
         assert (re.iterations, re.refinements) == (r.iterations, r.refinements), rid
+
+
+@pytest.mark.parametrize("inner", ["fp32", "fp64"])
+def test_fused_and_block_forms_same_bits(inner):
+    """Batches on both sides of the fused form's limit (592 chunks with FP32 inner solves, 296 with
+    FP64): small meshes of odd lengths beside one that just fits, beside one just past it (the block
+    form) and alone have the same bits; the large meshes those of their single solves in FP32, on both
+    sides of the single solver's limit."""
+    edge = {"fp32": (serving.Request(20, 72, 72, 73), serving.Request(21, 72, 72, 76)),
+            "fp64": (serving.Request(20, 57, 57, 56), serving.Request(21, 57, 57, 62))}[inner]
+    small = {i: serving.prepare(serving.Request(i, *size))  # under one chunk, just over one, several
+             for i, size in enumerate(((6, 4, 9), (8, 6, 11), (10, 10, 13)))}
+
+    def eng():
+        return fx.BatchEngine(1 << 21, 8, options=fx.SolveOptions(relative_tolerance=RTOL), inner=inner)
+
+    want = {}
+    for rid, (force, b, n) in small.items():
+        assert n % 2
+        e = eng()
+        want[rid] = run_to_end(e, {e.admit(force, b): rid})[rid]
+    extra = sum(-(-n // 2048) for _, _, n in small.values())
+    limit = {"fp32": 592, "fp64": 296}[inner]
+    for i, req in enumerate(edge):
+        force, b, n = serving.prepare(req)
+        chunks = -(-n // 2048)
+        assert (chunks + extra <= limit) if i == 0 else (chunks > limit)
+        e = eng()
+        slots = {e.admit(force, b): req.id}
+        slots.update({e.admit(f, bs): rid for rid, (f, bs, _) in small.items()})
+        got = run_to_end(e, slots, ticks=4000)
+        for rid in small:
+            assert np.array_equal(got[rid][0], want[rid][0]), (rid, chunks)
+        assert got[req.id][1].converged
+        if inner == "fp32":
+            x, r = single_ir(force, b, n)
+            assert np.array_equal(got[req.id][0], x) and r.iterations == got[req.id][1].iterations
 
 
 def test_alone_and_in_mix_are_the_same(prepared, alone):

@@ -4,8 +4,9 @@ recurrence in numpy on the oracle's operator, for vectors of less than one chunk
 one, odd lengths and many chunks, lane counts 1, 7 and 32, and a solution vector off the pairs'
 16-byte alignment. The two differ by rounding: each of the k iterations forms its products and sums
 with relative errors of a few n eps, so 1e-11 of the largest entry bounds them, and a chunk or an
-entry left out shows at 1e-4 and above. The same solve in one batch and alone, and in batches past
-the fused form's size, has the same bits (test_gpu_nbatch.py)."""
+entry left out shows at 1e-4 and above. The same at the largest vector that the fused form takes and
+just past it. In FP32, and in every form, a solve has the same bits alone and in a batch
+(test_gpu_batch.py, test_gpu_nbatch.py)."""
 import numpy as np
 import pytest
 
@@ -56,6 +57,24 @@ def test_iterates(size, oracle_mod):
                 got.append(x.cpu().numpy())
             assert np.max(np.abs(got[0] - want)) <= 1e-11 * np.max(np.abs(want)), (lanes, k)
             assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("size", [(57, 57, 60), (57, 57, 62)], ids=["largest_fused", "past_it"])
+def test_iterates_at_the_limit(size, oracle_mod):
+    mesh = fx.Model(meshes.box_model(*size)).compile().mesh()
+    n = mesh.num_equations
+    chunks = -(-n // 2048)
+    assert chunks == {60: 296, 62: 306}[size[2]]  # 2 blocks on each of 148 SMs: 296 fit
+    force, port = fx.InternalForce(mesh), oracle_mod.PortMesh(mesh)
+    b = np.random.default_rng(1).standard_normal(n)
+    d = torch.zeros(n, dtype=torch.float64, device=DEV)
+    force.operator_diagonal(fx.OperatorCoefficients(), d)
+    want = reference(port, b, d.cpu().numpy(), 3)
+    s = fx.ConjugateGradient(fx.SolveOptions(relative_tolerance=1e-30, max_iterations=3))
+    s.setup(fx.MatrixFreeOperator(force))
+    x = torch.zeros(n, dtype=torch.float64, device=DEV)
+    assert s.solve(torch.as_tensor(b, device=DEV), x).iterations == 3
+    assert np.max(np.abs(x.cpu().numpy() - want)) <= 1e-11 * np.max(np.abs(want))
 
 
 def test_infinite_alpha():

@@ -2,8 +2,9 @@
 hardening and loads on one cyclic load path in one batch. Each instance's displacement history
 and Newton solve counts must be bit for bit those of the single-instance path (fx_solver_newton
 with the same options) on that mesh alone: the combined mesh keeps every instance's gather order,
-and every instance's reductions run over its own range in the documented order, in the
-block-per-chunk form of the CG kernels (few chunks) and the warp-per-chunk form (more than 1,024).
+and every instance's reductions run over its own range in the documented order, in the fused form
+of the CG iteration (batches whose chunks fit on the GPU at once), the block-per-chunk form of its
+kernels and the warp-per-chunk form (more than 1,024 chunks).
 """
 import numpy as np
 import pytest
@@ -81,7 +82,7 @@ def test_mixed_batched_newton_equals_single_mixed_paths():
 def test_many_instances_warp_form_equals_single_paths():
     """More than 1,024 instances: the combined mesh spans more than 1,024 chunks (each instance's
     range padded to whole chunks), so the batch's CG vector kernels take the warp-per-chunk form,
-    while each instance alone (one chunk) takes the block-per-chunk form: the same bits."""
+    while each instance alone (one chunk) takes the fused form: the same bits."""
     inst = instances()
     count = 1030
     meshes, loads, mons = [], [], []
@@ -97,6 +98,32 @@ def test_many_instances_warp_form_equals_single_paths():
     for i in (0, 5, 517, count - 1):
         single = stages.load_path(fx.InternalForce(meshes[i]), torch.as_tensor(loads[i], device=DEV), factors,
                                   mons[i], tol=1e-6)
+        assert np.array_equal(batched.monitor[:, i], single.monitor), i
+        assert np.array_equal(batched.newton[:, i], single.newton), i
+        assert single.converged, i
+    assert batched.converged
+
+
+@pytest.mark.parametrize("count,mixed", [(296, False), (297, False), (592, True), (593, True)],
+                         ids=["fp64_fused", "fp64_block", "fp32_fused", "fp32_block"])
+def test_instances_on_both_sides_of_the_fused_limit(count, mixed):
+    """Batches of as many chunks (one per instance) as fit on the GPU at once (FP64 296, FP32 592) take
+    the fused form, one more the block-per-chunk form: the bits of the single paths either way."""
+    inst = instances()
+    meshes, loads, mons = [], [], []
+    for i in range(count):
+        mesh, F, mon = inst[i % len(inst)]
+        meshes.append(mesh)
+        loads.append(F * (0.6 + 0.4 * (i % 7) / 6.0))
+        mons.append(mon)
+    assert fx.BatchedNewton(meshes).offsets[-1] // 2048 == count
+    factors = stages.cyclic_factors(1, 8)[:2]
+    batched = stages.batched_load_path(meshes, loads, factors, mons, tol=1e-6, mixed=mixed)
+    for i in (0, 5, count // 2 + 2, count - 1):
+        solver = fx.MixedPrecisionSolver(fx.SolveOptions(relative_tolerance=1e-12, max_iterations=20000),
+                                         inner_tolerance=1e-4) if mixed else None
+        single = stages.load_path(fx.InternalForce(meshes[i]), torch.as_tensor(loads[i], device=DEV), factors,
+                                  mons[i], tol=1e-6, solver=solver)
         assert np.array_equal(batched.monitor[:, i], single.monitor), i
         assert np.array_equal(batched.newton[:, i], single.newton), i
         assert single.converged, i

@@ -269,3 +269,42 @@ def test_critical_dt_matches_reference(oracle_mod, ref_available):
         rf = oracle_mod.RefForce(oracle_mod.RefModel(spec).compile())
         for scheme in ("ExplicitDifference", "CentralDifference"):
             assert abs(force.min_critical_dt(scheme) - rf.min_critical_dt(scheme)) <= 1e-10 * rf.min_critical_dt(scheme)
+
+
+@pytest.mark.parametrize("path", ["box", "general"])
+@pytest.mark.parametrize("steps", [1, 2, 3, 16, 17, 18, 19, 33, 34, 35])
+def test_explicit_run_lengths(steps, path, oracle_mod):
+    """explicit_run where its graphs of 16 steps begin and end (the acceleration is written on a call's
+    last two steps and each graph's last, the step counter advanced once per graph): displacement,
+    velocities, acceleration and record of one call, and of two calls that continue each other, within
+    1e-10 of the oracle's; in FP32 within 2e-3."""
+    spec, _ = meshes.layered_box(6, 5, 4, layers=4, seed=6, h=1.0)
+    mesh, force, c = build(spec)
+    force.set_path(path)
+    eq_dof = c.array("eq_dof").astype(np.int8)
+    dt = 0.5 * force.min_critical_dt("ExplicitDifference")
+    n = mesh.num_equations
+    ag = np.random.default_rng(steps).uniform(0.5, 1.0, steps)
+    *want, hist = oracle_mod.PortMesh(mesh).ed_steps(mesh.lumped_mass, eq_dof, dt, steps, ag=ag, direction=0,
+                                                     record_eq=n - 1)
+
+    def run(parts, dtype):
+        state = [torch.zeros(n, dtype=dtype, device=DEV) for _ in range(4)]  # u, vh, a, v
+        got, at = [], 0
+        for k in parts:
+            got.append(force.explicit_run(t(mesh.lumped_mass, dtype), *state, dt, k, ag=ag[at:at + k], direction=0,
+                                          record_eq=n - 1))
+            at += k
+        return [s.double().cpu().numpy() for s in state], np.concatenate(got)
+
+    first = steps // 2
+    for parts in ((steps,), (first, steps - first) if first else (steps,)):
+        state, h = run(parts, torch.float64)
+        for name, got, ref in zip(("u", "vh", "a", "v"), state, want):
+            assert np.max(np.abs(got - ref)) <= 1e-10 * np.max(np.abs(ref)), (name, parts)
+        assert np.max(np.abs(h - hist)) <= 1e-10 * np.max(np.abs(hist)), parts
+        if path == "box":
+            state, h = run(parts, torch.float32)
+            for name, got, ref in zip(("u", "vh", "a", "v"), state, want):
+                assert np.max(np.abs(got - ref)) <= 2e-3 * np.max(np.abs(ref)), (name, parts)
+            assert np.max(np.abs(h - hist)) <= 2e-3 * np.max(np.abs(hist)), parts
