@@ -704,7 +704,10 @@ __device__ __forceinline__ T slot_sum_warp(const int32_t* __restrict__ list, con
 // kernels of internal_force.cpp:368-375, 442-448, same expression, same order). The first `hblocks`
 // blocks take the equations heavy[0 .. nheavy) (more than kHeavySlots slots each: tied DOFs) a warp
 // each, so that their long sums start first and overlap the others; the other blocks a thread per
-// equation, leaving the heavy ones.
+// equation, leaving the heavy ones. HEAVY: the mesh has such equations. Their sums take the kernel from 32
+// registers to 48, so a mesh without them runs the other form (B200, each call of a small mesh's operator,
+// force or diagonal 2 us less, the diagonal at 60^3 208 -> 199 us).
+template <bool HEAVY>
 __global__ void __launch_bounds__(256) k_gather(const int32_t* __restrict__ start, const int32_t* __restrict__ list,
                                                  const double* __restrict__ slots, int32_t neq,
                                                  const int32_t* __restrict__ heavy, int32_t nheavy, int32_t hblocks,
@@ -715,7 +718,7 @@ __global__ void __launch_bounds__(256) k_gather(const int32_t* __restrict__ star
   if (skip && *skip) return;
   double sum;
   int32_t q;
-  if (static_cast<int32_t>(blockIdx.x) < hblocks) {
+  if (HEAVY && static_cast<int32_t>(blockIdx.x) < hblocks) {
     const int32_t w = static_cast<int32_t>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (w >= nheavy) return;  // (the same for the whole warp)
     q = heavy[w];
@@ -733,14 +736,17 @@ __global__ void __launch_bounds__(256) k_gather(const int32_t* __restrict__ star
   y[q] = sum;
 }
 
+int32_t heavy_blocks(const ForceState& s) {
+  return static_cast<int32_t>(s.nheavy > 0 ? grid_for(32 * static_cast<int64_t>(s.nheavy), 256) : 0);
+}
+
 // y = every equation's slot sum and nodal terms (one k_gather launch)
 void gather_slots(const ForceState& s, double c1, const double* m1, const double* x1, double c2, const double* m2,
                   const double* x2, double* y, const int* skip, cudaStream_t st) {
   if (s.neq <= 0) return;
-  const int32_t hblocks = static_cast<int32_t>(s.nheavy > 0 ? grid_for(32 * static_cast<int64_t>(s.nheavy), 256) : 0);
-  k_gather<<<hblocks + grid_for(s.neq, 256), 256, 0, st>>>(s.gstart.ptr, s.glist.ptr, s.slots.ptr, s.neq,
-                                                           s.gheavy.ptr, s.nheavy, hblocks, c1, m1, x1, c2, m2, x2, y,
-                                                           skip);
+  const int32_t hblocks = heavy_blocks(s);
+  (hblocks ? k_gather<true> : k_gather<false>)<<<hblocks + grid_for(s.neq, 256), 256, 0, st>>>(
+      s.gstart.ptr, s.glist.ptr, s.slots.ptr, s.neq, s.gheavy.ptr, s.nheavy, hblocks, c1, m1, x1, c2, m2, x2, y, skip);
 }
 
 // ---- FP32 operator (the inner solves of FP32 CG in FP64 refinement on any mesh)
@@ -850,6 +856,7 @@ __global__ void __launch_bounds__(kBlock) k_element_apply32(const int32_t* __res
   for (int a = 0; a < 24; ++a) slots[static_cast<int64_t>(a) * P + e] = ye[a];
 }
 
+template <bool HEAVY>
 __global__ void __launch_bounds__(256) k_gather32(const int32_t* __restrict__ start, const int32_t* __restrict__ list,
                                                    const float* __restrict__ slots, int32_t neq,
                                                    const int32_t* __restrict__ heavy, int32_t nheavy, int32_t hblocks,
@@ -859,7 +866,7 @@ __global__ void __launch_bounds__(256) k_gather32(const int32_t* __restrict__ st
   if (skip && *skip) return;
   float sum;
   int32_t q;
-  if (static_cast<int32_t>(blockIdx.x) < hblocks) {  // the heavy equations, a warp each (as k_gather)
+  if (HEAVY && static_cast<int32_t>(blockIdx.x) < hblocks) {  // the heavy equations, a warp each (as k_gather)
     const int32_t w = static_cast<int32_t>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (w >= nheavy) return;
     q = heavy[w];
@@ -1125,11 +1132,11 @@ void general_apply_f32(ForceState& s, const double k[3], const float* x, float* 
   FX_LAUNCH_CHECK("element_apply32");
   const double* m1 = (k[2] != 0.0 && s.has_nodal_mass) ? s.nodal_mass.ptr : nullptr;
   const double* m2 = (k[1] != 0.0 && s.has_nodal_alpha) ? s.nodal_alpha_mass.ptr : nullptr;
+  const int32_t hblocks = heavy_blocks(s);
   if (s.neq > 0)
-    k_gather32<<<(s.nheavy > 0 ? grid_for(32 * static_cast<int64_t>(s.nheavy), 256) : 0) + grid_for(s.neq, 256), 256, 0,
-                 st>>>(s.gstart.ptr, s.glist.ptr, s.slots32.ptr, s.neq, s.gheavy.ptr, s.nheavy,
-                       static_cast<int32_t>(s.nheavy > 0 ? grid_for(32 * static_cast<int64_t>(s.nheavy), 256) : 0),
-                       k[2], m1, k[1], m2, x, y, skip);
+    (hblocks ? k_gather32<true> : k_gather32<false>)<<<hblocks + grid_for(s.neq, 256), 256, 0, st>>>(
+        s.gstart.ptr, s.glist.ptr, s.slots32.ptr, s.neq, s.gheavy.ptr, s.nheavy, hblocks, k[2], m1, k[1], m2, x, y,
+        skip);
   FX_LAUNCH_CHECK("slot_gather32");
 }
 
