@@ -1164,11 +1164,32 @@ void general_force_gather(ForceState& s, const double* v, double* f, cudaStream_
   FX_LAUNCH_CHECK("slot_gather");
 }
 
+// Whether the exact operator takes the point-parallel kernel (k_points_apply) or a thread per element
+// (k_element_apply: the same bits); the latter alone knows SSPbrick and soil sets. With the mass term
+// the points win at every size (49,321 bricks 58 -> 41 us, 60^3 181 -> 164). Without it a thread per
+// element is faster where its waves of 37,888 elements are well filled, as eight points cost more
+// FP64 work than one element's shared loops: about 11.5 us a wave against 4.2 us for one of 9,472
+// (B200, K x with the gather, thread per element against points: 30^3 23.5, 22.8; 33^3 23.9, 26.9; 34^3
+// 33.0, 28.9; 38^3 33.0, 35.2; 48^3 53.7, 65.6; 60^3 105, 129; 75^3 193, 244). J2 sets lean on the
+// points' parallelism for the dense sums of plastic tangents up to about 100,000 elements (96,000: 68.0,
+// 63.8 plastic, 68.1, 57.5 elastic; 128,000: 85, 90 plastic, 85, 77 elastic; 300,000: 176, 201 and 176,
+// 181).
+bool points_apply_pays(const ForceState& s, bool mass) {
+  if (s.has_ssp || s.has_pimy || s.has_pdmy) return false;
+  if (mass) return true;
+  if (s.has_j2) return s.count <= 100000;
+  const int64_t per_element = 2 * kBlock * static_cast<int64_t>(num_sms());  // elements of a wave
+  const int64_t per_point = 2 * points::kEl * static_cast<int64_t>(num_sms());
+  const int64_t we = (s.count + per_element - 1) / per_element, wp = (s.count + per_point - 1) / per_point;
+  return 4 * wp <= 11 * we + 1;
+}
+
 void general_apply(ForceState& s, const double k[3], const double* x, double* y, cudaStream_t st, const int* skip) {
   refuse_pimy_initial(s);
   if (general_fast_applies(s)) return general_apply_fast(s, k, x, y, st, skip);
-  if (s.count > 0 && !s.has_ssp && !s.has_pimy && !s.has_pdmy) {  // every set an elastic or J2 stdBrick set
-    if (k[2] != 0.0 || (k[1] != 0.0 && s.any_alpha)) launch_points_apply<true>(s, k, x, st, skip);
+  const bool mass = k[2] != 0.0 || (k[1] != 0.0 && s.any_alpha);
+  if (s.count > 0 && points_apply_pays(s, mass)) {
+    if (mass) launch_points_apply<true>(s, k, x, st, skip);
     else launch_points_apply<false>(s, k, x, st, skip);
   } else if (s.count > 0) {
     k_element_apply<<<grid_for(s.count, kBlock), kBlock, 0, st>>>(s.coords.ptr, s.node.ptr, s.eq.ptr, s.param.ptr,

@@ -67,6 +67,31 @@ def test_j2_sets(size, oracle_mod):
                 assert np.array_equal(got, port.apply_j2(D, k, x, initial=initial)), (amplitude, k, initial)
 
 
+@pytest.mark.parametrize("n", [30, 31, 36, 38])  # point-parallel, a thread per element, and both again
+def test_stiffness_only_on_both_sides_of_the_rule(n, oracle_mod):
+    mesh = fx.Model(meshes.distort(meshes.box_model(n, n, n), 0.1, seed=n)).compile().mesh()
+    force, port = fx.InternalForce(mesh), oracle_mod.PortMesh(mesh)
+    x = np.random.default_rng(n).standard_normal(mesh.num_equations)
+    got = apply(force, mesh.num_equations, fx.OperatorCoefficients(), x)
+    assert np.array_equal(got, port.apply_operator((1.0, 0.0, 0.0), x))
+
+
+@pytest.mark.parametrize("size", [(37, 37, 73), (37, 37, 74)])  # below and above 100,000 elements
+def test_j2_stiffness_on_both_sides_of_the_rule(size, oracle_mod):
+    mesh = fx.Model(j2_column(*size)).compile().mesh()
+    assert abs(mesh.count - 100000) < 1500
+    force, port = fx.InternalForce(mesh), oracle_mod.PortMesh(mesh)
+    n = mesh.num_equations
+    rng = np.random.default_rng(6)
+    u = 2e-3 * rng.standard_normal(n)
+    f = torch.zeros(n, dtype=torch.float64, device=DEV)
+    force.compute(torch.as_tensor(u, device=DEV), torch.zeros_like(f), f)
+    _, _, D, npl = port.force_j2(port.j2_state(), u, np.zeros(n))
+    assert npl > 0
+    x = rng.standard_normal(n)
+    assert np.array_equal(apply(force, n, fx.OperatorCoefficients(), x), port.apply_j2(D, (1.0, 0.0, 0.0), x))
+
+
 @pytest.mark.parametrize("size", [(16, 15, 2), (17, 16, 2), (33, 32, 2)])  # tied rows below and above 256 slots
 def test_tied_dofs(size, oracle_mod):
     mesh = fx.Model(soil_column(*size)).compile().mesh()
