@@ -296,6 +296,7 @@ int fx_force_create(const fx_mesh* mesh, int32_t device, fx_force** out) {
         p.betaK = q.betaK;
         p.betaKinit = q.betaKinit;
         p.betaKcomm = q.betaKcomm;
+        s.any_beta = s.any_beta || q.betaK != 0.0 || q.betaKinit != 0.0 || q.betaKcomm != 0.0;
         p.mass_type = q.mass_type;
         p.kind = q.kind;
         p.sigma_y = q.sigma_y;

@@ -19,6 +19,7 @@ DEV = torch.device("cuda:0")
 MESHES = {
     "distorted": lambda: meshes.distort(meshes.box_model(7, 5, 6, lumped=False), 0.25, seed=9),
     "column_ties": lambda: soil_column(4, 3, 10),
+    "undamped_body": lambda: meshes.distort(meshes.box_model(9, 4, 5, b=(0.3, -0.2, -9.8)), 0.2, seed=5),
     "block_damped": lambda: meshes.distort(two_region_block(6, 5, 7), 0.1, seed=2),
     "hetero": lambda: meshes.distort(meshes.heterogeneous_cube(5, seed=3), 0.15, seed=4),
 }
