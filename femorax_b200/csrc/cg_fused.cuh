@@ -182,7 +182,7 @@ __device__ __forceinline__ Sums iterate(const Chunk<T>& a) {
         vr[k] = fma(-alpha, va[k], vr[k]);
         vi[k] = vi[k] * vr[k];
       }
-      if (a.len < kChunk)  // (an infinite alpha makes the zeros past the end NaN)
+      if (!(fabs(alpha) < INFINITY))  // (it made NaN of the zeros past the chunk's end)
 #pragma unroll
         for (int k = 0; k < kChunkPer; ++k)
           if (pair_at(k / 2) + k % 2 >= a.len) vr[k] = vi[k] = T(0);
