@@ -233,7 +233,7 @@ struct ForceState {
   // value k of element e at [k * P + e] (ssp_brick.cuh: kGeo, kCon values)
   bool has_ssp = false;
   // the Gauss-point path's form: exact (false: the reference's arithmetic order, bit for bit) or
-  // fast (true: eight threads per element, fused multiply-adds; elastic stdBrick sets only)
+  // fast (true: a thread per Gauss point, fused multiply-adds; elastic stdBrick sets only)
   bool fast_general = false;
   DeviceArray<double> ssp_geo, ssp_con;
   // stable time step: the minimum's key (general.cu) and, for the periodic re-check, each

@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(kBlock) k_soil_force(const double* __restrict_
 
 // The same, point-parallel (points.cuh), where no set carries damping: element_force_from_stress's sums
 // in its order, per point the stress term and then minus the body force, which the sum forms from the
-// point's volume. 64,000 elements, B200: 43 -> 24 us (a thread per element held 255 registers).
+// point's volume. 64,000 elements, B200: 44 -> 40 us (a thread per element held 255 registers).
 __global__ void __launch_bounds__(points::kThreads, 2)
     k_soil_force_points(const double* __restrict__ coords, const int32_t* __restrict__ node,
                         const int32_t* __restrict__ eq, const int32_t* __restrict__ param,
@@ -665,8 +665,8 @@ __device__ __forceinline__ T slot_sum(const int32_t* __restrict__ list, const T*
 // The same sum by one warp, for equations with many slots (a tied DOF gathers whole rows of
 // elements): 256 slots loaded at once, the next 256 on their way while these are added in list order
 // by every lane. The 640 slots of a tied DOF of the 40^3 laminar column are then one chain of
-// additions: the gather launch takes 17 us there instead of 33 (32 slots at a time, each batch
-// waiting for its list entries and then its slots).
+// additions: the gather launch takes 17 us there instead of 34, with warm caches 15 instead of 24 (32
+// slots at a time, each batch waiting for its list entries and then its slots).
 template <class T>
 __device__ __forceinline__ T slot_sum_warp(const int32_t* __restrict__ list, const T* __restrict__ slots, int32_t j0,
                                            int32_t j1) {
@@ -1166,7 +1166,7 @@ void general_force_gather(ForceState& s, const double* v, double* f, cudaStream_
 
 // Whether the exact operator takes the point-parallel kernel (k_points_apply) or a thread per element
 // (k_element_apply: the same bits); the latter alone knows SSPbrick and soil sets. With the mass term
-// the points win at every size (49,321 bricks 58 -> 41 us, 60^3 181 -> 164). Without it a thread per
+// the points win at every size (49,321 bricks 51 -> 37 us, 60^3 with the gather 181 -> 164). Without it a thread per
 // element is faster where its waves of 37,888 elements are well filled, as eight points cost more
 // FP64 work than one element's shared loops: about 11.5 us a wave against 4.2 us for one of 9,472
 // (B200, K x with the gather, thread per element against points: 30^3 23.5, 22.8; 33^3 23.9, 26.9; 34^3

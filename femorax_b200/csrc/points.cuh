@@ -7,8 +7,10 @@
 // What bounds these kernels is latency at 16 warps per SM (128 registers), the FP64 pipe at 46 % of
 // its rate (about 5,200 operations per element without the mass term). A thread per element (before)
 // held 255 registers, 8 warps per SM, and its eight points ran one after the other. Measured, B200:
-// the exact operator with mass on 49,321 distorted bricks 58 -> 41 us, on 5,120 J2 bricks 22.2 ->
-// 7.1 us, on 15,700 J2 bricks 22.4 -> 12.4 us; the fast force on 64,000 bricks 55 -> 53 us.
+// caches warm: the exact operator with mass on 49,321 distorted bricks 51.1 -> 36.8 us, on 5,120 J2
+// bricks 17.5 -> 7.1 us, on 15,700 J2 bricks 17.5 -> 11.9 us; the damped fast force on 64,000 bricks
+// 46.1 -> 46.9 us (the undamped one 39 us with the gather; general_fast.cu). A thread per element stays
+// where it is faster: points_apply_pays in general.cu.
 #pragma once
 
 #include "force.hpp"

@@ -373,8 +373,10 @@ __device__ void cg_beta_step(double* sc, int* fl) {
 }
 
 // CG iterations per pass of the loop graph: fewer body relaunches (11.8 ms a 32^3 solve with 8, 12.1 with
-// 4, 12.7 with 2, before the fused iteration's arrivals were moved) and condition kernels against
-// at most kCgPass - 1 empty iterations after the solve ends.
+// 4, 12.7 with 2, before the fused iteration's arrivals were moved; 256 iterations at 3.06 M equations,
+// three vector kernels each, 33.4 ms with 8, 33.6 with 4) and condition kernels against at most
+// kCgPass - 1 empty iterations after the solve ends (7.9 us each there, so a solve of 9 to 12 iterations
+// is 1 % longer than with 4).
 constexpr int kCgPass = 8;
 
 // The loop graph's condition as the fused iteration sets it (after the last iteration of a pass).

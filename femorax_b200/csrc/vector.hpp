@@ -46,8 +46,9 @@ __device__ __forceinline__ void lane_loop(int64_t begin, int64_t len, int lane, 
 constexpr int kChunkBlock = 256;
 constexpr int kChunkPer = static_cast<int>(kChunk) / kChunkBlock;
 // Vectors past the fused CG iteration's size (cg_fused.cuh) and of at most this many chunks use the
-// block-per-chunk forms; longer ones keep a warp per chunk (enough warps in flight already; measured on a B200: the block forms 1.4x faster at 64 and
-// 51 chunks, equal at 1,495, 4-7 % slower at the served engine's thousands of chunks).
+// block-per-chunk forms; longer ones keep a warp per chunk (enough warps in flight already; measured
+// on a B200: the block forms 1.4x faster at 64 and 51 chunks, equal at 1,495, 4-7 % slower at the
+// served engine's thousands of chunks).
 constexpr int64_t kBlockChunks = 1024;
 
 // A chunk's sum of a[j] * b[j], j < len (a, b in shared memory), by one warp: lane l accumulates
