@@ -298,6 +298,7 @@ int fx_force_create(const fx_mesh* mesh, int32_t device, fx_force** out) {
         p.betaKcomm = q.betaKcomm;
         s.any_beta = s.any_beta || q.betaK != 0.0 || q.betaKinit != 0.0 || q.betaKcomm != 0.0;
         p.mass_type = q.mass_type;
+        s.any_consistent = s.any_consistent || q.mass_type == 0;
         p.kind = q.kind;
         p.sigma_y = q.sigma_y;
         p.H = q.H;

@@ -188,6 +188,7 @@ struct ForceState {
   bool has_nodal_mass = false, has_nodal_alpha = false;
   bool any_alpha = false;  // a parameter set with mass-proportional damping
   bool any_beta = false;   // a parameter set with stiffness-proportional damping
+  bool any_consistent = false;  // a parameter set with the consistent mass
   bool all_soil = false;   // every parameter set bound to a multi-yield soil
   int path = FX_PATH_AUTO;  // requested
   uint64_t forms = 0;       // counts the calls that change which kernels or buffers the operator runs on

@@ -1165,18 +1165,19 @@ void general_force_gather(ForceState& s, const double* v, double* f, cudaStream_
 }
 
 // Whether the exact operator takes the point-parallel kernel (k_points_apply) or a thread per element
-// (k_element_apply: the same bits); the latter alone knows SSPbrick and soil sets. With the mass term
-// the points win at every size (49,321 bricks 51 -> 37 us, 60^3 with the gather 181 -> 164). Without it a thread per
-// element is faster where its waves of 37,888 elements are well filled, as eight points cost more
-// FP64 work than one element's shared loops: about 11.5 us a wave against 4.2 us for one of 9,472
-// (B200, K x with the gather, thread per element against points: 30^3 23.5, 22.8; 33^3 23.9, 26.9; 34^3
-// 33.0, 28.9; 38^3 33.0, 35.2; 48^3 53.7, 65.6; 60^3 105, 129; 75^3 193, 244). J2 sets lean on the
-// points' parallelism for the dense sums of plastic tangents up to about 100,000 elements (96,000: 68.0,
-// 63.8 plastic, 68.1, 57.5 elastic; 128,000: 85, 90 plastic, 85, 77 elastic; 300,000: 176, 201 and 176,
-// 181).
+// (k_element_apply: the same bits); the latter alone knows SSPbrick and soil sets. With the consistent
+// mass term the points win at every size (49,321 bricks 51 -> 37 us, 60^3 with the gather 181 -> 164).
+// Without it, or with lumped masses only, a thread per element is faster where its waves of 37,888
+// elements are well filled, as eight points cost more FP64 work than one element's shared loops: about
+// 11.5 us a wave against 4.2 us for one of 9,472. B200, with the gather, thread per element against points:
+// K x 30^3 23.5, 22.8; 33^3 23.9, 26.9; 34^3 33.0, 28.9; 38^3 33.0, 35.2; 48^3 53.7, 65.6; 60^3 105, 129;
+// 75^3 193, 244; lumped 33^3 28.9, 33.0; 34^3 41.2, 35.1; 38^3 43.6, 43.3; 48^3 68.0, 81.2; 75^3 248, 301.
+// J2 sets lean on the points' parallelism for the dense sums of plastic tangents up to about 100,000
+// elements (K x 96,000: 68.0, 63.8 plastic, 68.1, 57.5 elastic; 128,000: 85, 90 plastic, 85, 77 elastic;
+// 300,000: 176, 201 and 176, 181; lumped 300,000: 215, 244 and 215, 222).
 bool points_apply_pays(const ForceState& s, bool mass) {
   if (s.has_ssp || s.has_pimy || s.has_pdmy) return false;
-  if (mass) return true;
+  if (mass && s.any_consistent) return true;
   if (s.has_j2) return s.count <= 100000;
   const int64_t per_element = 2 * kBlock * static_cast<int64_t>(num_sms());  // elements of a wave
   const int64_t per_point = 2 * points::kEl * static_cast<int64_t>(num_sms());

@@ -67,13 +67,16 @@ def test_j2_sets(size, oracle_mod):
                 assert np.array_equal(got, port.apply_j2(D, k, x, initial=initial)), (amplitude, k, initial)
 
 
+@pytest.mark.parametrize("lumped", [False, True], ids=["consistent", "lumped"])
 @pytest.mark.parametrize("n", [30, 31, 36, 38])  # point-parallel, a thread per element, and both again
-def test_stiffness_only_on_both_sides_of_the_rule(n, oracle_mod):
-    mesh = fx.Model(meshes.distort(meshes.box_model(n, n, n), 0.1, seed=n)).compile().mesh()
+def test_operator_on_both_sides_of_the_rule(n, lumped, oracle_mod):
+    """K x, and with the mass term: its consistent form is point-parallel at every size."""
+    mesh = fx.Model(meshes.distort(meshes.box_model(n, n, n, lumped=lumped), 0.1, seed=n)).compile().mesh()
     force, port = fx.InternalForce(mesh), oracle_mod.PortMesh(mesh)
-    x = np.random.default_rng(n).standard_normal(mesh.num_equations)
-    got = apply(force, mesh.num_equations, fx.OperatorCoefficients(), x)
-    assert np.array_equal(got, port.apply_operator((1.0, 0.0, 0.0), x))
+    for k in ((1.0, 0.0, 0.0), (1.0, 0.0, 3.0)):
+        x = np.random.default_rng(n).standard_normal(mesh.num_equations)
+        got = apply(force, mesh.num_equations, fx.OperatorCoefficients(*k), x)
+        assert np.array_equal(got, port.apply_operator(k, x)), k
 
 
 @pytest.mark.parametrize("size", [(37, 37, 73), (37, 37, 74)])  # below and above 100,000 elements
